@@ -34,6 +34,15 @@ struct PolyH {
   double max_rel_error = 0.0;
 };
 
+// FP64 coefficients of H(t) in s = t*scale - 1 on [0, t_cut]; terms 0: no fit
+// reaches FP64 accuracy (very large r_cut / r_s).
+constexpr int kPoly64Short = 20, kPoly64Max = 32;
+struct PolyH64 {
+  int terms = 0;
+  double scale = 0.0;
+  double c[kPoly64Max] = {};
+};
+
 // Per-solve scalar geometry shared with the walk kernel.
 struct WalkParams {
   double box[3];
@@ -68,6 +77,7 @@ struct Context {
   int device = 0;
   double spacing = 0.0, rs = 0.0, cutoff = 0.0;
   PolyH poly;
+  PolyH64 poly64;  // H(t) for FP64 pairs
   PolyH dpoly;   // H'(t): the adjoint walk and FP32 multipoles
   PolyH ddpoly;  // H''(t): FP32 quadrupoles
   std::string last_error;
@@ -123,6 +133,7 @@ struct Context {
   DevBuf sort_hist, sort_counts, sort_totals, sort_keys, sort_vals;
   int64_t n_nodes = 0;
   uint32_t max_depth = 0;
+  double root_half = 0.0;  // half-size of the root node
   int path_words_used = 0;
   int unwrap_sorted_axes = 0;  // axes whose unwrap sorted the coordinates (bit a)
   int prev_tree_depth = 0;     // depth of the previous tree built by this context (0: none)
@@ -153,7 +164,8 @@ struct Context {
   // walk
   DevBuf walk_counters;  // 8 x u64
   DevBuf walk_cost;      // per 32 visit positions: SM cycles of the last walk (float)
-  DevBuf work_counter;   // u32 dynamic scheduling
+  DevBuf work_counter;   // u32 dynamic scheduling, group-walk groups, target groups
+  DevBuf walk_groups;    // {first visit position, targets} of each group of targets
   DevBuf tree_acc;       // double3 per active slot (short-range part)
   DevBuf tree_near;      // double per active slot
   // the production walk counts its traversal and pairs and records the

@@ -1025,6 +1025,7 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
   const double cy0 = 0.5 * (lo[1] + hi[1]);
   const double cz0 = 0.5 * (lo[2] + hi[2]);
   const double half0 = 0.5 * mext * (1.0 + 1.0e-8);
+  c.root_half = half0;
   int depth_half = 0;
   for (double h = half0; !(h <= 1.0e-12) && depth_half < 4 * kMaxDepth; h *= 0.5) ++depth_half;
 

@@ -1,0 +1,124 @@
+"""The strict policy's production walk where its groups, images and batches can
+go wrong: fewer targets than a warp, remainders, meshes so coarse that a pair's
+other image is in reach, targets spread over the box, coincident particles,
+explicit targets, softening lanes, and the sizes around the walk's choice of
+lanes per target -- against the FP64 oracle."""
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+
+import chui_treepm as ct  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+BOX = (10.0, 9.0, 11.0)
+
+
+@pytest.fixture(autouse=True)
+def cuda_ok():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+def particles(n, seed):
+    """A third uniform, the rest in blobs, one of them across the box corner;
+    two coincident particles."""
+    rng = np.random.default_rng(seed)
+    L = np.array(BOX)
+    x = rng.uniform(0.0, 1.0, (n, 3)) * L
+    for k, c in enumerate(([0.02, 0.97, 0.01], [0.4, 0.5, 0.6])):
+        rows = np.arange(n) % 3 == k + 1
+        x[rows] = np.array(c) * L + rng.normal(0.0, 0.25, (int(rows.sum()), 3))
+    x = np.mod(x, L)
+    if n > 4:
+        x[n // 2] = x[n // 3]
+    m = rng.uniform(0.5, 2.0, n)
+    return x[:, 0].copy(), x[:, 1].copy(), x[:, 2].copy(), m
+
+
+def config(mesh, precision, **kw):
+    return ct.TreePmConfig(pm_grid_nx=mesh, pm_grid_ny=mesh, pm_grid_nz=mesh, box_x=BOX[0], box_y=BOX[1], box_z=BOX[2],
+                           opening_theta=0.6, max_leaf_size=16, softening=0.05, precision=precision, **kw)
+
+
+def reference(p, mesh, active=None, quadrupole=1):
+    o = oracle.treepm_solve(*p, oracle.make_params(box=BOX, mesh=(mesh,) * 3, theta=0.6, eps=0.05, leaf=16,
+                                                   quadrupole=quadrupole), active=active)
+    return np.stack([o["ax"], o["ay"], o["az"]])
+
+
+def off(r, ref):
+    got = np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")])
+    assert np.isfinite(got).all()
+    return np.abs(got - ref).max() / np.abs(ref).max()
+
+
+# FP32 pairs: the long-range polynomial is within 5e-5 of its part of each pair
+# and the largest accelerations are sums of pairs of their own size
+MIXED = 1.0e-4
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 257, 3000])
+@pytest.mark.parametrize("mesh", [14, 20, 48])
+def test_small_boxes_and_remainders(n, mesh):
+    p = particles(n, n + mesh)
+    with ct.TreePmCoordinator(config(mesh, ct._abi.MIXED)) as s:
+        r = s.solve_active_set(*p)
+    if n == 1:
+        # no pairs: the mesh's own force, zero up to its FP32 rounding (about
+        # 1e-7 of the deposited particle's force scale m / r_s^2)
+        rs = 1.25 * (BOX[0] * BOX[1] * BOX[2]) ** (1 / 3) / mesh
+        assert max(abs(r[k][0]) for k in ("ax", "ay", "az")) <= 1e-6 * p[3][0] / rs ** 2
+        return
+    assert off(r, reference(p, mesh)) <= MIXED
+    # monopole order 0: nothing is accepted, every pair is summed
+    with ct.TreePmCoordinator(config(mesh, ct._abi.FP64, multipole_order=0)) as s:
+        r = s.solve_active_set(*p)
+    assert off(r, reference(p, mesh, quadrupole=0)) <= 1e-11
+
+
+@pytest.mark.parametrize("count", [1, 5, 40, 333])
+@pytest.mark.parametrize("mesh", [16, 40])
+def test_sparse_and_explicit_targets(count, mesh):
+    p = particles(2500, 7)
+    act = np.random.default_rng(count).permutation(2500)[:count].astype(np.uint32)
+    ref = reference(p, mesh, active=act)
+    with ct.TreePmCoordinator(config(mesh, ct._abi.MIXED)) as s:
+        assert off(s.solve_active_set(*p, active=act), ref) <= MIXED
+        # the same targets given by position, a box length away on two axes
+        t = (p[0][act] + BOX[0], p[1][act], p[2][act] - BOX[2])
+        assert off(s.solve_active_set(*p, active=act, targets=t), ref) <= MIXED
+    with ct.TreePmCoordinator(config(mesh, ct._abi.FP64, multipole_order=0)) as s:
+        ref = reference(p, mesh, active=act, quadrupole=0)
+        assert off(s.solve_active_set(*p, active=act), ref) <= 1e-11
+        assert off(s.solve_active_set(*p, active=act, targets=t), ref) <= 1e-11
+
+
+@pytest.mark.parametrize("n", [4735, 4736, 32001, 64005, 128031])
+def test_lanes_per_target(n):
+    """The sizes on both sides of each change of the lanes sharing a target:
+    mixed against the FP64 walk (itself against the oracle above)."""
+    p = particles(n, n)
+    t = [torch.tensor(v, device="cuda") for v in p]
+    out = {}
+    for prec in (ct._abi.MIXED, ct._abi.FP64):
+        with ct.TreePmCoordinator(config(48, prec)) as s:
+            r = s.solve_active_set(*t)
+            out[prec] = torch.stack([r[k] for k in ("ax", "ay", "az")])
+    d = (out[ct._abi.MIXED] - out[ct._abi.FP64]).abs().max() / out[ct._abi.FP64].abs().max()
+    assert float(d) <= MIXED
+
+
+@pytest.mark.parametrize("r_cut", [6.25, 9.0, 14.0])
+def test_fp64_long_range_coefficient(r_cut):
+    """r_cut / r_s of 5, 7.2 and 11.2: the 20-term and 32-term polynomials and
+    the closed form of the FP64 pairs."""
+    p = particles(600, 3)
+    with ct.TreePmCoordinator(config(48, ct._abi.FP64, multipole_order=0, rcut_cells=r_cut)) as s:
+        r = s.solve_active_set(*p)
+    o = oracle.treepm_solve(*p, oracle.make_params(box=BOX, mesh=(48,) * 3, rcut=r_cut, theta=0.6, eps=0.05, leaf=16,
+                                                   quadrupole=0))
+    assert off(r, np.stack([o["ax"], o["ay"], o["az"]])) <= 1e-11
