@@ -1378,9 +1378,9 @@ int chui_treepm_force_vjp(void* handle, const chui_treepm_sources* src, const do
       (rc = chui::stageIn(c, c.in_tz, cot_z, n, memory, s, &cz)))
     return rc;
   if (!src->mass) m = nullptr;
-  double lo[3], hi[3], mass_sum = 0.0;
+  double lo[3], hi[3], mass_sum = 0.0, mass_range[2] = {0.0, 0.0};
   uint32_t st = 0;
-  if ((rc = chui::sourceBounds(c, n, x, y, z, m, lo, hi, &mass_sum, &st, s))) return rc;
+  if ((rc = chui::sourceBounds(c, n, x, y, z, m, lo, hi, &mass_sum, &st, s, mass_range))) return rc;
   if (st) return chui::fail(c, CHUI_TREEPM_EINVAL, "TreePM sources require finite coordinates and finite non-negative masses");
   const double total_mass = m ? mass_sum : static_cast<double>(n) * src->uniform_mass;
   double *gx = grad_x, *gy = grad_y, *gz = grad_z;
@@ -1425,7 +1425,10 @@ int chui_treepm_force_vjp(void* handle, const chui_treepm_sources* src, const do
   if (n > 0) {
     if (chui::ensure(c.tree_acc, static_cast<size_t>(n) * 3 * 8)) return chui::fail(c, CHUI_TREEPM_ENOMEM, "allocation failed");
     double* t = c.tree_acc.as<double>();
-    if ((rc = chui::walkVjpRun(c, n, x, y, z, m, src->uniform_mass, cx, cy, cz, wp, t, t + n, t + 2 * n, s)))
+    // equal masses travel as one value
+    const bool equal_masses = m && mass_range[0] == mass_range[1];
+    if ((rc = chui::walkVjpRun(c, n, x, y, z, equal_masses ? nullptr : m,
+                               equal_masses ? mass_range[0] : src->uniform_mass, cx, cy, cz, wp, t, t + n, t + 2 * n, s)))
       return chui::fail(c, rc, "adjoint walk launch failed");
     cudaEventRecord(c.ev[3], s);
     { chui::noteLaunch(); chui::addKernel<<<chui::gridFor(n, 256), 256, 0, s>>>(n, gx, gy, gz, t); }

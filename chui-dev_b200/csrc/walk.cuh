@@ -438,6 +438,124 @@ __device__ __forceinline__ int certainLess(float a, float b, float err = 0.f) {
   return 0;
 }
 
+// order-preserving signed integer image of a float
+__device__ __forceinline__ int floatOrder(float f) {
+  const int i = __float_as_int(f);
+  return i ^ ((i >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float fromFloatOrder(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
+
+// The group's centre to FP32: offsets of nearby FP64 positions from it are
+// exact, so a pair's separation is rounded once.
+__device__ __forceinline__ double coarse(double v) {
+  const float f = static_cast<float>(v);
+  return isfinite(f) ? static_cast<double>(f) : v;
+}
+
+constexpr int kBatchStack = 224;         // stack entries beyond the depth-first bound, for nodes taken together
+constexpr float kFar = 1.0e15f;          // padding entry of a source queue, outside every cutoff
+constexpr uint32_t kWideRun = 1u << 31;  // group record: the 32 visit positions around it spread wide
+
+// The box of a warp's targets (FP64 positions, one per lane, near each other
+// in one frame): centre and half extents, rounding included.
+struct GroupFrame {
+  double cx, cy, cz;
+  float hx, hy, hz;
+};
+
+__device__ __forceinline__ void groupAxis(double p, float off, double& c, float& h) {
+  const float lo = fromFloatOrder(__reduce_min_sync(0xffffffffu, floatOrder(off)));
+  const float hi = fromFloatOrder(__reduce_max_sync(0xffffffffu, floatOrder(off)));
+  c = coarse(p + static_cast<double>(0.5f * (lo + hi)));
+  const float mid = static_cast<float>(c - p);
+  h = fmaxf(hi - mid, mid - lo) + 3.0e-7f * (hi - lo + fabsf(mid));
+}
+
+__device__ __forceinline__ GroupFrame groupFrame(double px, double py, double pz, bool valid) {
+  GroupFrame f;
+  const double rx = __shfl_sync(0xffffffffu, px, 0), ry = __shfl_sync(0xffffffffu, py, 0),
+               rz = __shfl_sync(0xffffffffu, pz, 0);
+  groupAxis(rx, valid ? static_cast<float>(px - rx) : 0.f, f.cx, f.hx);
+  groupAxis(ry, valid ? static_cast<float>(py - ry) : 0.f, f.cy, f.hy);
+  groupAxis(rz, valid ? static_cast<float>(pz - rz) : 0.f, f.cz, f.hz);
+  return f;
+}
+
+// One node per lane against the box of the targets: the nearest image of its
+// centre (whole box lengths k, offset nd), the squared distance from the box
+// to the cube's nearest point (low side of rounding) and the squared reach of
+// all targets to its farthest corner (high side).
+struct NodeReach {
+  uint4 rg;
+  double half;
+  double kx, ky, kz, ndx, ndy, ndz;
+  float ax, ay, az, hf, gap2, far2;
+};
+
+__device__ __forceinline__ NodeReach nodeReach(const double4* __restrict__ geom, const uint4* __restrict__ range,
+                                               uint32_t node, bool have, const GroupFrame& f, const WalkParams& w) {
+  NodeReach r;
+  double4 g = make_double4(0.0, 0.0, 0.0, 0.0);
+  r.rg = make_uint4(0u, 0u, 0u, 0u);
+  if (have) {
+    g = geom[node];
+    r.rg = range[node];
+  }
+  r.half = g.w;
+  // L = 0: no images
+  r.kx = w.box[0] > 0.0 ? rint((g.x - f.cx) * w.inv_box[0]) : 0.0;
+  r.ky = w.box[1] > 0.0 ? rint((g.y - f.cy) * w.inv_box[1]) : 0.0;
+  r.kz = w.box[2] > 0.0 ? rint((g.z - f.cz) * w.inv_box[2]) : 0.0;
+  r.ndx = (g.x - f.cx) - w.box[0] * r.kx;
+  r.ndy = (g.y - f.cy) - w.box[1] * r.ky;
+  r.ndz = (g.z - f.cz) - w.box[2] * r.kz;
+  r.hf = __double2float_ru(g.w);
+  r.ax = fabsf(static_cast<float>(r.ndx));
+  r.ay = fabsf(static_cast<float>(r.ndy));
+  r.az = fabsf(static_cast<float>(r.ndz));
+  const float gx = fmaxf(fmaf(r.ax, 0.9999995f, -(r.hf + f.hx)), 0.f), gy = fmaxf(fmaf(r.ay, 0.9999995f, -(r.hf + f.hy)), 0.f),
+              gz = fmaxf(fmaf(r.az, 0.9999995f, -(r.hf + f.hz)), 0.f);
+  r.gap2 = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+  const float wx = r.ax + r.hf + f.hx, wy = r.ay + r.hf + f.hy, wz = r.az + r.hf + f.hz;
+  r.far2 = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
+  return r;
+}
+
+// The children of the lanes' nodes that are opened (push) go on the stack, each
+// with `flag` set; returns the new height, or sets overflow.
+__device__ __forceinline__ int pushChildren(const uint32_t* __restrict__ child, uint32_t node, bool push,
+                                            uint32_t children, uint32_t flag, uint32_t* stack, int sp, int cap,
+                                            bool& overflow, uint32_t* stack_mask = nullptr, uint32_t mask = 0u) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = push ? children : 0u;
+  uint32_t incl = n;
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+  if (sp + static_cast<int>(total) > cap) {
+    overflow = true;
+    return sp;
+  }
+  if (push) {
+    uint32_t at = static_cast<uint32_t>(sp) + incl - n;
+    const uint4* ch = reinterpret_cast<const uint4*>(child + 8 * static_cast<size_t>(node));
+    const uint4 c0 = ch[0], c1 = ch[1];
+    const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {
+      if (c[o] != kInvalid) {
+        stack[at] = c[o] | flag;
+        if (stack_mask) stack_mask[at] = mask;
+        ++at;
+      }
+    }
+  }
+  __syncwarp();
+  return sp + static_cast<int>(total);
+}
+
 }  // namespace
 
 // Groups of at most `most` (a power of two, <= 32) nearby targets over the

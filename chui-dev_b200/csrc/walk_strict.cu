@@ -60,9 +60,7 @@ constexpr uint32_t kStrictCull = 512;
 // queued sources per batch (128: 2 % slower at 256^3)
 constexpr int kQueue32 = 256;
 constexpr int kQueue64 = 128;
-constexpr int kBatchStack = 224;      // stack entries beyond the depth-first bound, for nodes taken together
 constexpr uint32_t kInBlock = 1u << 31;  // stack entry inside a subtree block (node ids stay below 2^31)
-constexpr float kFar = 1.0e15f;       // padding entry, outside every cutoff
 
 // Resident blocks per SM the FP32 registers are sized for. 4, 5 and 6 (128, 96
 // and 80 registers) are equal to 1 % (160.9 / 160.9 / 161.8 ms at 256^3), 7 and
@@ -71,16 +69,7 @@ constexpr float kFar = 1.0e15f;       // padding entry, outside every cutoff
 // where two or more warps evaluate (the loop alone, measured with 2 to 8).
 constexpr int kBlocks32 = 5;
 
-constexpr uint32_t kWideRun = 1u << 31;  // group record: the 32 visit positions around it spread wide
-
 enum SourceLanes { kUniformMass = 0, kMassLane = 1, kMassEpsLanes = 2 };
-
-// order-preserving signed integer image of a float
-__device__ __forceinline__ int floatOrder(float f) {
-  const int i = __float_as_int(f);
-  return i ^ ((i >> 31) & 0x7fffffff);
-}
-__device__ __forceinline__ float fromFloatOrder(int i) { return __int_as_float(i ^ ((i >> 31) & 0x7fffffff)); }
 
 // A target's position: its source's tree-frame position, or the explicit one.
 __device__ __forceinline__ void targetPosition(const WalkArgs& a, int64_t v, uint32_t slot, uint32_t row, double& x,
@@ -95,13 +84,6 @@ __device__ __forceinline__ void targetPosition(const WalkArgs& a, int64_t v, uin
     y = u.y;
     z = u.z;
   }
-}
-
-// The group's centre to FP32: offsets of nearby FP64 positions from it are
-// exact, so a pair's separation is rounded once.
-__device__ __forceinline__ double coarse(double v) {
-  const float f = static_cast<float>(v);
-  return isfinite(f) ? static_cast<double>(f) : v;
 }
 
 // Offset of a target from a point near it. Tree-frame positions are unwrapped:
@@ -261,29 +243,17 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       }
     }
     const uint32_t self_pos = kIndex && valid && row < a.n ? a.pos_of_row[row] : kInvalid;
-    // the box of the targets: centre and half extents (a bound: rounding included)
-    double cx = __shfl_sync(0xffffffffu, ux, 0), cy = __shfl_sync(0xffffffffu, uy, 0),
-           cz = __shfl_sync(0xffffffffu, uz, 0);
-    float hbx, hby, hbz;
+    // the box of the targets
+    GroupFrame frame;
     {
-      const float fx = valid ? static_cast<float>(targetOffset(a, ux - cx, 0)) : 0.f;
-      const float fy = valid ? static_cast<float>(targetOffset(a, uy - cy, 1)) : 0.f;
-      const float fz = valid ? static_cast<float>(targetOffset(a, uz - cz, 2)) : 0.f;
-      const float lx = fromFloatOrder(__reduce_min_sync(0xffffffffu, floatOrder(fx)));
-      const float ux = fromFloatOrder(__reduce_max_sync(0xffffffffu, floatOrder(fx)));
-      const float ly = fromFloatOrder(__reduce_min_sync(0xffffffffu, floatOrder(fy)));
-      const float uy = fromFloatOrder(__reduce_max_sync(0xffffffffu, floatOrder(fy)));
-      const float lz = fromFloatOrder(__reduce_min_sync(0xffffffffu, floatOrder(fz)));
-      const float uz = fromFloatOrder(__reduce_max_sync(0xffffffffu, floatOrder(fz)));
-      const double rx = cx, ry = cy, rz = cz;
-      cx = coarse(rx + static_cast<double>(0.5f * (lx + ux)));
-      cy = coarse(ry + static_cast<double>(0.5f * (ly + uy)));
-      cz = coarse(rz + static_cast<double>(0.5f * (lz + uz)));
-      const float mx = static_cast<float>(cx - rx), my = static_cast<float>(cy - ry), mz = static_cast<float>(cz - rz);
-      hbx = fmaxf(ux - mx, mx - lx) + 3.0e-7f * (ux - lx + fabsf(mx));
-      hby = fmaxf(uy - my, my - ly) + 3.0e-7f * (uy - ly + fabsf(my));
-      hbz = fmaxf(uz - mz, mz - lz) + 3.0e-7f * (uz - lz + fabsf(mz));
+      const double rx = __shfl_sync(0xffffffffu, ux, 0), ry = __shfl_sync(0xffffffffu, uy, 0),
+                   rz = __shfl_sync(0xffffffffu, uz, 0);
+      groupAxis(rx, valid ? static_cast<float>(targetOffset(a, ux - rx, 0)) : 0.f, frame.cx, frame.hx);
+      groupAxis(ry, valid ? static_cast<float>(targetOffset(a, uy - ry, 1)) : 0.f, frame.cy, frame.hy);
+      groupAxis(rz, valid ? static_cast<float>(targetOffset(a, uz - rz, 2)) : 0.f, frame.cz, frame.hz);
     }
+    const double cx = frame.cx, cy = frame.cy, cz = frame.cz;
+    const float hbx = frame.hx, hby = frame.hy, hbz = frame.hz;
     // the origin of the FP32 offsets: the centre, or the first target of a run of
     // 32 that spreads wide (its pairs keep the rounding of that frame)
     double fx0 = cx, fy0 = cy, fz0 = cz;
@@ -499,70 +469,27 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       __syncwarp();
       const uint32_t node = entry & ~kInBlock;
       bool in_block = (entry & kInBlock) != 0u;
-      double4 g = make_double4(0.0, 0.0, 0.0, 0.0);
-      uint4 rg = make_uint4(0u, 0u, 0u, 0u);
-      if (have) {
-        g = a.geom[node];
-        rg = a.range[node];
-      }
-      // nearest image of the node centre (L = 0: no images)
-      const double kx = w.box[0] > 0.0 ? rint((g.x - cx) * w.inv_box[0]) : 0.0;
-      const double ky = w.box[1] > 0.0 ? rint((g.y - cy) * w.inv_box[1]) : 0.0;
-      const double kz = w.box[2] > 0.0 ? rint((g.z - cz) * w.inv_box[2]) : 0.0;
-      const double ndx = (g.x - cx) - w.box[0] * kx, ndy = (g.y - cy) - w.box[1] * ky, ndz = (g.z - cz) - w.box[2] * kz;
-      const float hf = __double2float_ru(g.w);
-      const float ax = fabsf(static_cast<float>(ndx)), ay = fabsf(static_cast<float>(ndy)), az = fabsf(static_cast<float>(ndz));
-      // distances from the box to the nearest point of the cube (low side of
-      // rounding) and of all targets to its farthest corner (high side)
-      const float gx = fmaxf(fmaf(ax, 0.9999995f, -(hf + hbx)), 0.f), gy = fmaxf(fmaf(ay, 0.9999995f, -(hf + hby)), 0.f),
-                  gz = fmaxf(fmaf(az, 0.9999995f, -(hf + hbz)), 0.f);
-      const bool reach = have && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= cut_hi2;
-      const float wx = ax + hf + hbx, wy = ay + hf + hby, wz = az + hf + hbz;
-      const float far2 = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
+      const NodeReach r = nodeReach(a.geom, a.range, node, have, frame, w);
+      const uint4 rg = r.rg;
+      const float hf = r.hf;
+      const bool reach = have && r.gap2 <= cut_hi2;
       const bool leaf = rg.z == 0u;
       // could some target accept the node as a multipole? It must lie inside
       // r_cut of the target and be narrower than 0.08 of its distance.
       bool may = false;
       if (reach && !leaf && !in_block && hf < never_half) {
-        const float nx = fmaxf(ax - hbx, 0.f) + hf, ny = fmaxf(ay - hby, 0.f) + hf, nz = fmaxf(az - hbz, 0.f) + hf;
-        may = fmaf(nx, nx, fmaf(ny, ny, nz * nz)) <= cut_hi2 && 4.0f * hf * hf < 0.00641f * far2;
+        const float nx = fmaxf(r.ax - hbx, 0.f) + hf, ny = fmaxf(r.ay - hby, 0.f) + hf, nz = fmaxf(r.az - hbz, 0.f) + hf;
+        may = fmaf(nx, nx, fmaf(ny, ny, nz * nz)) <= cut_hi2 && 4.0f * hf * hf < 0.00641f * r.far2;
       }
-      if (!may && !leaf && rg.y <= kStrictBlock && g.w <= sa.block_half) in_block = true;
-      const bool whole = leaf || (in_block && (rg.y <= kStrictCull || far2 <= cut_lo2));
+      if (!may && !leaf && rg.y <= kStrictBlock && r.half <= sa.block_half) in_block = true;
+      const bool whole = leaf || (in_block && (rg.y <= kStrictCull || r.far2 <= cut_lo2));
       const bool emit = reach && !may && whole;
       const bool push = reach && !may && !whole;
 
       // children of the opened nodes
-      {
-        const uint32_t n_child = push ? rg.z : 0u;
-        uint32_t incl = n_child;
-        for (int off = 1; off < 32; off <<= 1) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, off);
-          if (lane >= off) incl += y;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        if (sp + static_cast<int>(total) > sa.stack_cap) {
-          overflow = true;
-          break;
-        }
-        if (push) {
-          uint32_t at = static_cast<uint32_t>(sp) + incl - n_child;
-          const uint32_t flag = in_block ? kInBlock : 0u;
-          const uint4* ch = reinterpret_cast<const uint4*>(a.child + 8 * static_cast<size_t>(node));
-          const uint4 c0 = ch[0], c1 = ch[1];
-          const uint32_t c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-#pragma unroll
-          for (int o = 0; o < 8; ++o) {
-            if (c[o] != kInvalid) {
-              stack[at] = c[o] | flag;
-              stack_mask[at] = mask;
-              ++at;
-            }
-          }
-        }
-        sp += static_cast<int>(total);
-        __syncwarp();
-      }
+      sp = pushChildren(a.child, node, push, rg.z, in_block ? kInBlock : 0u, stack, sp, sa.stack_cap, overflow,
+                        stack_mask, mask);
+      if (overflow) break;
 
       // nodes some target may accept: decided per target (every lane, one node
       // at a time); the rest of the targets see the node again, opened
@@ -572,8 +499,8 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
         const uint32_t lanes = __shfl_sync(0xffffffffu, mask, j);
         const double4 ng = a.geom[nd];
         const uint4 nr = a.range[nd];
-        const double ox = __shfl_sync(0xffffffffu, ndx, j), oy = __shfl_sync(0xffffffffu, ndy, j),
-                     oz = __shfl_sync(0xffffffffu, ndz, j);
+        const double ox = __shfl_sync(0xffffffffu, r.ndx, j), oy = __shfl_sync(0xffffffffu, r.ndy, j),
+                     oz = __shfl_sync(0xffffffffu, r.ndz, j);
         bool accept = false;
         if (valid && ((lanes >> lane) & 1u)) {
           float mx = 0.f, my = 0.f, mz = 0.f;  // COM offset of an accepted node
@@ -700,31 +627,32 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       const float Lx = static_cast<float>(w.box[0]), Ly = static_cast<float>(w.box[1]), Lz = static_cast<float>(w.box[2]);
       // reach of the group spans more than the nearest image on some axis
       const float rc = sa.cut_f * 1.00001f + hf;
-      const bool images = emit && ((Lx > 0.f && ax + hbx + rc >= Lx * 0.99999f) || (Ly > 0.f && ay + hby + rc >= Ly * 0.99999f) ||
-                                   (Lz > 0.f && az + hbz + rc >= Lz * 0.99999f));
-      const unsigned moved = __ballot_sync(0xffffffffu, emit && (kx != 0.0 || ky != 0.0 || kz != 0.0));
+      const bool images = emit && ((Lx > 0.f && r.ax + hbx + rc >= Lx * 0.99999f) ||
+                                   (Ly > 0.f && r.ay + hby + rc >= Ly * 0.99999f) ||
+                                   (Lz > 0.f && r.az + hbz + rc >= Lz * 0.99999f));
+      const unsigned moved = __ballot_sync(0xffffffffu, emit && (r.kx != 0.0 || r.ky != 0.0 || r.kz != 0.0));
       const unsigned many = __ballot_sync(0xffffffffu, images);
       for (unsigned todo = __ballot_sync(0xffffffffu, emit); todo; todo &= todo - 1u) {
         const int j = __ffs(todo) - 1;
         const uint32_t begin = __shfl_sync(0xffffffffu, rg.x, j), count = __shfl_sync(0xffffffffu, rg.y, j);
         const uint32_t lanes = __shfl_sync(0xffffffffu, mask, j);
         const bool shift = ((moved >> j) & 1u) != 0u, each = ((many >> j) & 1u) != 0u;
-        double jx = 0.0, jy = 0.0, jz = 0.0, ox = 0.0, oy = 0.0, oz = 0.0, r = 0.0;
+        double jx = 0.0, jy = 0.0, jz = 0.0, ox = 0.0, oy = 0.0, oz = 0.0, rr = 0.0;
         if (shift || each) {
-          jx = __shfl_sync(0xffffffffu, kx, j);
-          jy = __shfl_sync(0xffffffffu, ky, j);
-          jz = __shfl_sync(0xffffffffu, kz, j);
+          jx = __shfl_sync(0xffffffffu, r.kx, j);
+          jy = __shfl_sync(0xffffffffu, r.ky, j);
+          jz = __shfl_sync(0xffffffffu, r.kz, j);
         }
         if (each) {
-          ox = __shfl_sync(0xffffffffu, ndx, j);
-          oy = __shfl_sync(0xffffffffu, ndy, j);
-          oz = __shfl_sync(0xffffffffu, ndz, j);
-          r = static_cast<double>(__shfl_sync(0xffffffffu, rc, j)) * 1.00001;
+          ox = __shfl_sync(0xffffffffu, r.ndx, j);
+          oy = __shfl_sync(0xffffffffu, r.ndy, j);
+          oz = __shfl_sync(0xffffffffu, r.ndz, j);
+          rr = static_cast<double>(__shfl_sync(0xffffffffu, rc, j)) * 1.00001;
         }
         for (int im = each ? 0 : 13; im < (each ? 27 : 14); ++im) {
           const int ix = im / 9 - 1, iy = im / 3 % 3 - 1, iz = im % 3 - 1;
-          if (each && (fabs(ox + ix * w.box[0]) > r + hbx || fabs(oy + iy * w.box[1]) > r + hby ||
-                       fabs(oz + iz * w.box[2]) > r + hbz))
+          if (each && (fabs(ox + ix * w.box[0]) > rr + hbx || fabs(oy + iy * w.box[1]) > rr + hby ||
+                       fabs(oz + iz * w.box[2]) > rr + hbz))
             continue;
           // the nearest image of a node around the group keeps the origin's bits
           // (a target's own entry stays at distance zero)

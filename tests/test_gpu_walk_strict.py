@@ -122,3 +122,22 @@ def test_fp64_long_range_coefficient(r_cut):
     o = oracle.treepm_solve(*p, oracle.make_params(box=BOX, mesh=(48,) * 3, rcut=r_cut, theta=0.6, eps=0.05, leaf=16,
                                                    quadrupole=0))
     assert off(r, np.stack([o["ax"], o["ay"], o["az"]])) <= 1e-11
+
+
+@pytest.mark.parametrize("equal", [True, False])
+@pytest.mark.parametrize("mesh", [14, 48])
+@pytest.mark.parametrize("n", [2, 33, 257, 5000])
+def test_force_vjp_groups(n, mesh, equal):
+    """The mixed adjoint walk (the same groups and images, equal masses as one
+    value) against the FP64 adjoint; the bar is the forward walk's."""
+    p = [torch.tensor(v, device="cuda") for v in particles(n, n + mesh)]
+    if equal:
+        p[3] = torch.full_like(p[3], 1.25)
+    g = torch.Generator(device="cpu").manual_seed(n)
+    cot = [torch.randn(n, generator=g, dtype=torch.float64).to("cuda") for _ in range(3)]
+    out = {}
+    for prec in (ct._abi.MIXED, ct._abi.FP64):
+        with ct.TreePmCoordinator(config(mesh, prec)) as s:
+            out[prec] = torch.stack(s.force_vjp(*p, *cot))
+    d = torch.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64]) / torch.linalg.norm(out[ct._abi.FP64])
+    assert float(d) <= MIXED
