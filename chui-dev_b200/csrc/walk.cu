@@ -649,7 +649,16 @@ __device__ __forceinline__ void exactLeafPairs(const WalkArgs& a, double4* stage
   }
 }
 
-// Mixed-precision walk (the product path).
+// Centre and half extent (rounding included) of the warp's targets on one axis.
+__device__ __forceinline__ void targetBox(bool valid, float off, float& c, float& h) {
+  const float o = valid ? off : 0.f;  // lane 0 is the origin
+  const float lo = fromFloatOrder(__reduce_min_sync(0xffffffffu, floatOrder(o)));
+  const float hi = fromFloatOrder(__reduce_max_sync(0xffffffffu, floatOrder(o)));
+  c = 0.5f * (lo + hi);
+  h = 0.5f * (hi - lo) + 1.0e-6f * (hi - lo);
+}
+
+// Mixed-precision walk of the adaptive policy, and the counting walks.
 //
 // Traversal order and every per-lane decision are those of the reference's
 // evaluateTargetAgainstLocalTree. Each warp works in one FP64 reference frame
@@ -744,17 +753,28 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
   while (true) {
     uint32_t cnt_visited = 0, cnt_accepted = 0, cnt_opened = 0, cnt_pairs = 0, cnt_pruned = 0, cnt_skips = 0,
              cnt_multi = 0, cnt_leaves = 0;
+    // the next 32 visit positions, or under the adaptive policy the next group of
+    // nearby targets
     uint32_t base = 0;
-    if (lane == 0) base = static_cast<uint32_t>(a.v0) + atomicAdd(a.work, 32u);
+    if (lane == 0) base = atomicAdd(a.work, kAdaptive ? 1u : 32u);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= a.v1) break;
+    int64_t end = a.v1;
+    if constexpr (kAdaptive) {
+      if (base >= *a.group_count) break;
+      const uint2 gr = a.groups[base];
+      base = gr.x;
+      end = static_cast<int64_t>(gr.x) + (gr.y & ~kWideRun);
+    } else {
+      base += static_cast<uint32_t>(a.v0);
+      if (base >= a.v1) break;
+    }
     if constexpr (kCost) {
       // reading the clock costs the walk ~1.5 % in code generation, so only
       // the instances behind a visit-range solve do it
       if (lane == 0) item_start_sm[warp] = clock64();
     }
     const int64_t v = static_cast<int64_t>(base) + lane;
-    const bool valid = v < a.v1;
+    const bool valid = v < end;
     uint32_t slot = 0, row = kInvalid;
     double& px = lane_sm[0][warp][lane];
     double& py = lane_sm[1][warp][lane];
@@ -798,6 +818,18 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
     const double cull2d = kF64 ? (w.cutoff + sqrt(rg2)) * (w.cutoff + sqrt(rg2)) * (1.0 + 1.0e-12) : 0.0;
     const float cull = static_cast<float>(w.cutoff + sqrt(rg2));
     const float cull2 = cull * cull * 1.0001f;
+    // adaptive: the box of the group's targets (centre, half extents) instead
+    float bx = 0.f, by = 0.f, bz = 0.f, hbx = 0.f, hby = 0.f, hbz = 0.f;
+    if constexpr (kAdaptive) {
+      targetBox(valid, tfx, bx, hbx);
+      targetBox(valid, tfy, by, hby);
+      targetBox(valid, tfz, bz, hbz);
+    }
+    auto boxGap2 = [&](float ex, float ey, float ez, float h) {
+      const float gx = fmaxf(fabsf(ex - bx) - (hbx + h), 0.f), gy = fmaxf(fabsf(ey - by) - (hby + h), 0.f),
+                  gz = fmaxf(fabsf(ez - bz) - (hbz + h), 0.f);
+      return fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+    };
     const float rga_f = static_cast<float>(rga);
     const bool skip_self = valid && row < a.n;
     const uint32_t self_pos = skip_self ? a.pos_of_row[row] : kInvalid;
@@ -1058,7 +1090,8 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
                             static_cast<float>(static_cast<double>(sv.y) + cdy),
                             static_cast<float>(static_cast<double>(sv.z) + cdz), sv.w);
           }
-          keep = fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)) <= cull2;
+          keep = kAdaptive ? boxGap2(e.x, e.y, e.z, 0.f) <= cut2 * 1.0001f
+                           : fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)) <= cull2;
         }
         const uint32_t keep_mask = __ballot_sync(0xffffffffu, keep);
         const int c = __popc(keep_mask);
@@ -1341,7 +1374,19 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
             continue;
           }
         }
-        const uint32_t ch = lane < 8 ? a.child[8 * static_cast<size_t>(node) + lane] : kInvalid;
+        uint32_t ch = lane < 8 ? a.child[8 * static_cast<size_t>(node) + lane] : kInvalid;
+        if constexpr (kAdaptive && !kDiag) {
+          // children beyond r_cut of every target are not visited at all (the
+          // nearest image of the cube, rounding on the low side)
+          if (ch != kInvalid) {
+            const double4 cg = a.geom[ch];
+            const float ex = static_cast<float>(frameImage(cg.x - rx - bx, w.box[0], inv_l[0])) + bx;
+            const float ey = static_cast<float>(frameImage(cg.y - ry - by, w.box[1], inv_l[1])) + by;
+            const float ez = static_cast<float>(frameImage(cg.z - rz - bz, w.box[2], inv_l[2])) + bz;
+            const float h = static_cast<float>(cg.w) * 1.00001f + 1.0e-6f * (fabsf(ex) + fabsf(ey) + fabsf(ez));
+            if (boxGap2(ex, ey, ez, h) > cut2 * 1.0001f) ch = kInvalid;
+          }
+        }
         const unsigned cmask = __ballot_sync(0xffffffffu, ch != kInvalid) & 0xFFu;
         const int nc = __popc(cmask);
         if (sp + nc > kStackCap) {
@@ -1375,7 +1420,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
       }
     }
     if constexpr (kCost) {
-      if (lane == 0) a.chunk_cost[base >> 5] = static_cast<float>(clock64() - item_start_sm[warp]);
+      if (lane == 0) atomicAdd(a.chunk_cost + (base >> 5), static_cast<float>(clock64() - item_start_sm[warp]));
     }
     __syncwarp();
   }
@@ -1599,6 +1644,17 @@ int walkRun(Context& c, int64_t nt, const uint32_t* active, const double* tx, co
     // lane (with subtree blocks: the production traversal)
     const bool diag = c.cfg.diagnostics == 1 || c.walk_instrument;
     const bool uniform = wp.uniform_mass != 0;
+    if (wp.policy == CHUI_TREEPM_POLICY_ADAPTIVE) {
+      // groups of at most 32 nearby targets; in a tiny box runs of 32 (the FP32
+      // frame's reach then sends their pairs to FP64)
+      double limit = INFINITY;
+      if (!tinyBox(wp, n)) {
+        limit = 1.5 * c.cutoff;
+        if (wp.box[0] > 0.0) limit = std::min(limit, 0.25 * std::min({wp.box[0], wp.box[1], wp.box[2]}));
+      }
+      if (int rc = targetGroups(c, a, 32, limit, &a.groups, &a.group_count, s)) return rc;
+      a.work = c.work_counter.as<uint32_t>();
+    }
     const int mode = wp.policy == CHUI_TREEPM_POLICY_ADAPTIVE ? (wp.group_walk ? 3 : 2)
                                                                : (wp.criterion == 2 && prev_acc ? 1 : 0);
     if (soft) {

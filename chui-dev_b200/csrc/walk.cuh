@@ -79,13 +79,14 @@ struct WalkArgs {
   // FP64 production walk counts and records nearest pairs -- instrument
   int blocks;
   int instrument;
+  // groups of nearby targets ({first visit position, targets}) and their number
+  const uint2* groups;
+  const uint32_t* group_count;
   WalkParams wp;
 };
 
 // The strict production walk's own arguments (walk_strict.cu).
 struct StrictArgs {
-  const uint2* groups;          // {first visit position, targets}
-  const uint32_t* group_count;
   int targets_per_group;        // at most; a power of two
   int stack_cap, batch_cap;     // stack entries, and those open to taking several nodes at once
   double block_half;            // largest half-size of a subtree block

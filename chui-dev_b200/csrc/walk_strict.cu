@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
   const float never_half = w.quadrupole ? sa.accept_half : 0.f;  // nodes from this half-size on are never accepted
   const float theta2 = static_cast<float>(w.theta * w.theta);
   const float env2 = 0.0064f;  // 0.08^2
-  const uint32_t groups = *sa.group_count;
+  const uint32_t groups = *a.group_count;
 
   while (true) {
     uint32_t item = 0;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
     if (item >= groups) break;
     long long started = 0;
     if (a.chunk_cost) started = clock64();
-    const uint2 gr = sa.groups[item];
+    const uint2 gr = a.groups[item];
     const int64_t v = static_cast<int64_t>(gr.x) + t;
     const bool valid = t < static_cast<int>(gr.y & ~kWideRun);
     uint32_t slot = 0, row = kInvalid;
@@ -734,7 +734,7 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
   // at 256^3 clustered.
   double limit = 1.5 * c.cutoff;
   if (a.wp.box[0] > 0.0) limit = std::min(limit, 0.25 * std::min({a.wp.box[0], a.wp.box[1], a.wp.box[2]}));
-  if (int rc = targetGroups(c, a, per, limit, &sa.groups, &sa.group_count, s)) return rc;
+  if (int rc = targetGroups(c, a, per, limit, &a.groups, &a.group_count, s)) return rc;
   const int depth_first = 1 + 7 * std::max<int>(static_cast<int>(c.max_depth), 1);
   sa.batch_cap = kBatchStack;
   sa.stack_cap = (kBatchStack + depth_first + 7 + 1) & ~1;  // even: 16-byte aligned warps
