@@ -434,8 +434,8 @@ PolyH64 fitPoly64(double t_cut) {
     p.scale = 2.0 / t_cut;
     for (int i = 0; i < m; ++i) p.c[i] = static_cast<double>(mono[i]);
     double err = 0.0;
-    for (int k = 0; k <= 1000; ++k) {
-      const double t = t_cut * k / 1000.0, s = std::fma(t, p.scale, -1.0);
+    for (int k = 0; k <= 96; ++k) {  // several points to each of the fit's oscillations
+      const double t = t_cut * k / 96.0, s = std::fma(t, p.scale, -1.0);
       double h = p.c[m - 1];
       for (int i = m - 2; i >= 0; --i) h = std::fma(h, s, p.c[i]);
       err = std::max(err, std::fabs(static_cast<double>(static_cast<long double>(h) - exactH(t))));
@@ -599,10 +599,9 @@ int sourceBounds(Context& c, int64_t n, const double* x, const double* y, const 
   if (n > 0)
     { noteLaunch(); sourceReduceKernel<<<std::min(gridFor(n, 256), kReduceBlocks), 256, 0, s>>>(n, x, y, z, m, sc, reinterpret_cast<double*>(sc + 6),
                                                        c.status.as<uint32_t>()); }
-  unsigned long long hb[10];
-  uint32_t st = 0;
-  cudaMemcpyAsync(hb, sc, sizeof(hb), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(&st, c.status.ptr, 4, cudaMemcpyDeviceToHost, s);
+  unsigned long long* hb = c.pinned;
+  cudaMemcpyAsync(hb, sc, sizeof(init), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(hb + 10, c.status.ptr, 4, cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return fail(c, CHUI_TREEPM_EDEVICE, "source reduction failed");
   for (int a = 0; a < 3; ++a) {
     lo[a] = n > 0 ? fromOrderedBits(hb[a]) : INFINITY;
@@ -611,7 +610,7 @@ int sourceBounds(Context& c, int64_t n, const double* x, const double* y, const 
   double ms;
   std::memcpy(&ms, &hb[6], 8);
   *mass_sum = ms;
-  *status_bits = st;
+  *status_bits = *reinterpret_cast<uint32_t*>(hb + 10);
   if (mass_range) {
     mass_range[0] = (m && n > 0) ? fromOrderedBits(hb[8]) : 0.0;
     mass_range[1] = (m && n > 0) ? fromOrderedBits(hb[9]) : 0.0;
@@ -792,7 +791,10 @@ int chui_treepm_create(const chui_treepm_config* cfg, void** handle) {
   c->device = cfg->device;
   chui::DeviceGuard guard(c->device);
   chui::applyConfig(*c, *cfg);
-  if (chui::ensure(c->status, 64) != cudaSuccess || chui::ensure(c->scalars, 64 * 8) != cudaSuccess) {
+  if (chui::ensure(c->status, 64) != cudaSuccess || chui::ensure(c->scalars, 64 * 8) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void**>(&c->pinned), 16 * 8, cudaHostAllocDefault) != cudaSuccess) {
+    chui::release(c->status);
+    chui::release(c->scalars);
     delete c;
     g_create_error = "device allocation failed";
     return CHUI_TREEPM_ENOMEM;
@@ -826,6 +828,7 @@ void chui_treepm_destroy(void* handle) {
                             &c->tree_acc, &c->tree_near, &c->walk_cost, &c->walk_groups, &c->out_lr[0], &c->out_lr[1],
                             &c->out_lr[2]};
     for (auto* b : bufs) chui::release(*b);
+    cudaFreeHost(c->pinned);
     if (c->events_ready)
       for (auto& e : c->ev) cudaEventDestroy(e);
     if (c->pipe_ready) {
@@ -1061,8 +1064,6 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
     if (c.last_error.empty()) c.last_error = "TreePM tree build failed";
     return rc;
   }
-  double nlo[3], nhi[3];
-  if ((rc = chui::treeNodeBounds(c, nlo, nhi, s))) return chui::fail(c, rc, "node bounds failed");
   if ((rc = chui::treeOrderTargets(c, nt, active, explicit_targets ? 1 : 0, n, s)))
     return chui::fail(c, rc, "target ordering failed");
   cudaEventRecord(c.ev[1], s);
@@ -1085,8 +1086,8 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
   for (int a = 0; a < 3; ++a) {
     wp.src_lo[a] = lo[a];
     wp.src_hi[a] = hi[a];
-    wp.node_lo[a] = nlo[a];
-    wp.node_hi[a] = nhi[a];
+    wp.node_lo[a] = c.node_lo[a];
+    wp.node_hi[a] = c.node_hi[a];
   }
   wp.rs = c.rs;
   wp.cutoff = c.cutoff;
@@ -1228,11 +1229,11 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
   }
   c.visit_count = nt;
   cudaEventRecord(c.ev[4], s);
-  uint32_t walk_status = 0;
-  cudaMemcpyAsync(&walk_status, c.status.ptr, 4, cudaMemcpyDeviceToHost, s);
-  unsigned long long counters[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  unsigned long long* counters = c.pinned;
+  for (int k = 0; k < 9; ++k) counters[k] = 0ull;
+  cudaMemcpyAsync(counters + 8, c.status.ptr, 4, cudaMemcpyDeviceToHost, s);
   if (n > 0 && nt > 0 && c.walk_counters.ptr)
-    cudaMemcpyAsync(counters, c.walk_counters.ptr, sizeof(counters), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(counters, c.walk_counters.ptr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
   if (memory == CHUI_TREEPM_HOST && nout > 0) {
     cudaMemcpyAsync(acc->accel_x, ax, nout * 8, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(acc->accel_y, ay, nout * 8, cudaMemcpyDeviceToHost, s);
@@ -1251,6 +1252,7 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
   }
   cudaError_t e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return chui::fail(c, CHUI_TREEPM_EDEVICE, std::string("CUDA error: ") + cudaGetErrorString(e));
+  const uint32_t walk_status = *reinterpret_cast<uint32_t*>(counters + 8);
   if (walk_status) return chui::fail(c, CHUI_TREEPM_ERANGE, chui::statusText(walk_status));
   chui_treepm_stats stt{};
   stt.visited_nodes = counters[0];

@@ -134,6 +134,8 @@ struct Context {
   int64_t n_nodes = 0;
   uint32_t max_depth = 0;
   double root_half = 0.0;  // half-size of the root node
+  double node_lo[3] = {}, node_hi[3] = {};  // bounds of node centres and COMs
+  unsigned long long* pinned = nullptr;     // 16 words of page-locked host memory for small results
   int path_words_used = 0;
   int unwrap_sorted_axes = 0;  // axes whose unwrap sorted the coordinates (bit a)
   int prev_tree_depth = 0;     // depth of the previous tree built by this context (0: none)
@@ -226,23 +228,22 @@ void pmDestroy(Context& c);
 int treeBuild(Context& c, int64_t n, const double* x, const double* y, const double* z,
               const double* m, double uniform_mass, const double src_lo[3], const double src_hi[3],
               cudaStream_t s);
-int treeNodeBounds(Context& c, double lo[3], double hi[3], cudaStream_t s);
 int treeOrderTargets(Context& c, int64_t nt, const uint32_t* active, int explicit_targets, int64_t n,
                      cudaStream_t s);
 
 // ---- sort and scan (sort.cu) ----
 // Stable LSD radix sorts by the low end_bit bits (8-bit digits; digits equal
-// for every key are skipped); kin and kout must differ.
+// for every key are skipped); kin and kout must differ. With begin_bit > 0 the
+// whole digits below it are known to be zero and the others are sorted without
+// looking (no counting pass, no wait for its result).
 int radixSortPairsU64(Context& c, const unsigned long long* kin, unsigned long long* kout, const uint32_t* vin,
-                      uint32_t* vout, int64_t n, int end_bit, cudaStream_t s);
+                      uint32_t* vout, int64_t n, int end_bit, cudaStream_t s, int begin_bit = 0);
 // batch (<= 3) independent keys-only sorts of n keys each, in the same launches
 int radixSortKeysU64(Context& c, int batch, const unsigned long long* const* kin, unsigned long long* const* kout,
                      int64_t n, int end_bit, cudaStream_t s);
 int radixSortPairsU32(Context& c, const uint32_t* kin, uint32_t* kout, const uint32_t* vin, uint32_t* vout,
                       int64_t n, int end_bit, cudaStream_t s);
 int exclusiveScanU32(Context& c, const uint32_t* in, uint32_t* out, int64_t n, cudaStream_t s);
-// Maximum of n values, returned to the host (synchronises the stream).
-int maxU32(Context& c, const uint32_t* in, int64_t n, uint32_t* result, cudaStream_t s);
 
 // ---- walk (walk.cu) ----
 // Targets are the visit positions [visit_begin, visit_end) of the nt targets

@@ -1,4 +1,4 @@
-// Stable LSD radix sort, exclusive scan and maximum for the tree build.
+// Stable LSD radix sort and exclusive scan for the tree build.
 //
 // The reference orders particles with a stable least-significant-digit radix
 // sort of 8-bit digits (radixSortMortonOrdering, tree_ordering.cpp:13-71; the
@@ -275,7 +275,7 @@ __global__ void CHUI_SORT_BOUNDS downsweepKernel(int64_t n, SortJob job, SortJob
 // vary in any of them (a pass over a constant digit keeps the order)
 template <class K>
 int radixSortBatch(Context& c, int batch, const K* const* kin, K* const* kout, const uint32_t* const* vin,
-                   uint32_t* const* vout, int64_t n, int end_bit, cudaStream_t s) {
+                   uint32_t* const* vout, int64_t n, int end_bit, cudaStream_t s, int begin_bit = 0) {
   if (n <= 0) return 0;
   if (n > 0xFFFFFFFFll || batch < 1 || batch > kMaxBatch) return CHUI_TREEPM_ERANGE;
   const int digits = (end_bit + 7) / 8;
@@ -299,30 +299,34 @@ int radixSortBatch(Context& c, int batch, const K* const* kin, K* const* kout, c
     }
   }
   // which digits vary
-  uint32_t* hist = c.sort_hist.as<uint32_t>();
-  cudaMemsetAsync(hist, 0, kMaxBatch * 8 * 256 * sizeof(uint32_t), s);
-  {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t want = (n + kSortThreads - 1) / kSortThreads;
-    const unsigned blocks = static_cast<unsigned>(want < 4 * sms ? want : 4 * sms);
-    noteLaunch();
-    digitHistogramKernel<K><<<dim3(blocks, batch), kSortThreads, 0, s>>>(n, src, digits, hist);
-  }
-  std::vector<uint32_t> h(static_cast<size_t>(batch) * 8 * 256);
-  cudaMemcpyAsync(h.data(), hist, h.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
   std::vector<int> shifts;
-  for (int d = 0; d < digits; ++d) {
-    bool varies = false;
-    for (int y = 0; y < batch; ++y) {
-      bool constant = false;
-      for (int v = 0; v < 256; ++v)
-        if (h[(static_cast<size_t>(y) * 8 + d) * 256 + v] == static_cast<uint32_t>(n)) constant = true;
-      varies = varies || !constant;
+  if (begin_bit > 0) {
+    for (int d = begin_bit / 8; d < digits; ++d) shifts.push_back(8 * d);
+  } else {
+    uint32_t* hist = c.sort_hist.as<uint32_t>();
+    cudaMemsetAsync(hist, 0, kMaxBatch * 8 * 256 * sizeof(uint32_t), s);
+    {
+      int dev = 0, sms = 148;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int64_t want = (n + kSortThreads - 1) / kSortThreads;
+      const unsigned blocks = static_cast<unsigned>(want < 4 * sms ? want : 4 * sms);
+      noteLaunch();
+      digitHistogramKernel<K><<<dim3(blocks, batch), kSortThreads, 0, s>>>(n, src, digits, hist);
     }
-    if (varies) shifts.push_back(8 * d);
+    std::vector<uint32_t> h(static_cast<size_t>(batch) * 8 * 256);
+    cudaMemcpyAsync(h.data(), hist, h.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
+    for (int d = 0; d < digits; ++d) {
+      bool varies = false;
+      for (int y = 0; y < batch; ++y) {
+        bool constant = false;
+        for (int v = 0; v < 256; ++v)
+          if (h[(static_cast<size_t>(y) * 8 + d) * 256 + v] == static_cast<uint32_t>(n)) constant = true;
+        varies = varies || !constant;
+      }
+      if (varies) shifts.push_back(8 * d);
+    }
   }
   const int passes = static_cast<int>(shifts.size());
   if (passes == 0) {
@@ -401,20 +405,11 @@ __global__ void scanAddKernel(int64_t n, uint32_t* out, const uint32_t* __restri
     out[i] += tile_sums[i / kScanTile];
 }
 
-__global__ void maxKernel(int64_t n, const uint32_t* __restrict__ in, uint32_t* out) {
-  uint32_t m = 0u;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    m = max(m, in[i]);
-  for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 }  // namespace
 
 int radixSortPairsU64(Context& c, const unsigned long long* kin, unsigned long long* kout, const uint32_t* vin,
-                      uint32_t* vout, int64_t n, int end_bit, cudaStream_t s) {
-  return radixSortBatch<unsigned long long>(c, 1, &kin, &kout, &vin, &vout, n, end_bit, s);
+                      uint32_t* vout, int64_t n, int end_bit, cudaStream_t s, int begin_bit) {
+  return radixSortBatch<unsigned long long>(c, 1, &kin, &kout, &vin, &vout, n, end_bit, s, begin_bit);
 }
 
 int radixSortKeysU64(Context& c, int batch, const unsigned long long* const* kin, unsigned long long* const* kout,
@@ -436,16 +431,6 @@ int exclusiveScanU32(Context& c, const uint32_t* in, uint32_t* out, int64_t n, c
   { noteLaunch(); scanSumsKernel<<<1, kSortThreads, 0, s>>>(tiles, sums); }
   { noteLaunch(); scanAddKernel<<<gridFor(n, 256), 256, 0, s>>>(n, out, sums); }
   return cudaGetLastError() == cudaSuccess ? 0 : CHUI_TREEPM_EDEVICE;
-}
-
-int maxU32(Context& c, const uint32_t* in, int64_t n, uint32_t* result, cudaStream_t s) {
-  *result = 0u;
-  if (n <= 0) return 0;
-  uint32_t* d = reinterpret_cast<uint32_t*>(c.scalars.as<unsigned long long>() + 14);
-  cudaMemsetAsync(d, 0, 4, s);
-  { noteLaunch(); maxKernel<<<std::min(gridFor(n, 256), kReduceBlocks), 256, 0, s>>>(n, in, d); }
-  cudaMemcpyAsync(result, d, 4, cudaMemcpyDeviceToHost, s);
-  return cudaStreamSynchronize(s) == cudaSuccess ? 0 : CHUI_TREEPM_EDEVICE;
 }
 
 }  // namespace chui

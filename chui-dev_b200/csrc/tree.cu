@@ -82,23 +82,126 @@ __device__ __forceinline__ uint32_t gapBucket(double v, double scale, uint32_t n
   return f >= static_cast<double>(nb) ? nb - 1u : static_cast<uint32_t>(f);
 }
 
+// The periodic axes of one unwrap, one per blockIdx.y.
+struct UnwrapAxes {
+  const double* in[3];
+  double* out[3];
+  double box[3], scale[3];
+  int canonical[3];
+};
+
+// One of the axes' values by blockIdx.y with constant indices (a dynamic index
+// into the kernel's parameter block would copy it to local memory).
+template <class T>
+__device__ __forceinline__ T pickAxis(const T (&v)[3], int k) {
+  return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]);
+}
+
 // The canonical coordinate of every particle, and per gap bucket the
 // smallest and largest value, as bits (non-negative doubles order like their
 // bits). A plain read first skips the atomics that cannot change the bucket
 // (a stale read only ever asks for an atomic that was not needed): particles
-// in row order often share a bucket across a warp.
-__global__ void canonicalBucketsKernel(int64_t n, const double* __restrict__ in, double box, int canonical,
-                                       double* out, double scale, uint32_t nb, unsigned long long* bmin,
+// in row order often share a bucket across a warp. Axis k of the launch is
+// axis first + blockIdx.y, its buckets at bmin + blockIdx.y * nb.
+__global__ void canonicalBucketsKernel(int64_t n, UnwrapAxes ax, int first, uint32_t nb, unsigned long long* bmin,
                                        unsigned long long* bmax) {
+  const int k = first + static_cast<int>(blockIdx.y);
+  const double* __restrict__ in = pickAxis(ax.in, k);
+  double* __restrict__ out = pickAxis(ax.out, k);
+  const double box = pickAxis(ax.box, k), scale = pickAxis(ax.scale, k);
+  const int canonical = pickAxis(ax.canonical, k);
+  bmin += static_cast<size_t>(blockIdx.y) * nb;
+  bmax += static_cast<size_t>(blockIdx.y) * nb;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const double v = canonicalCoordinate(in[i], box, canonical);
     out[i] = v;
-    const uint32_t k = gapBucket(v, scale, nb);
-    const unsigned long long b = dbits(v);
-    if (b < bmin[k]) atomicMin(bmin + k, b);
-    if (b > bmax[k]) atomicMax(bmax + k, b);
+    const uint32_t b = gapBucket(v, scale, nb);
+    const unsigned long long bits = dbits(v);
+    if (bits < bmin[b]) atomicMin(bmin + b, bits);
+    if (bits > bmax[b]) atomicMax(bmax + b, bits);
   }
+}
+
+// Up to kGapBlockBuckets buckets an axis: the largest circular gap between
+// consecutive non-empty buckets, the anchor after it and the suspect flag (as
+// runGapKernel finds them over the compacted list) by one block per axis, in
+// one launch instead of seven. Each thread owns consecutive buckets and learns
+// the first value after them from a suffix scan over the block. One block reads
+// its axis's buckets twice at 100 to 200 GB/s; beyond kGapBlockBuckets that
+// costs more than the launches (tree build of 32 k particles 0.54 -> 0.36 ms with
+// the other steps of this kind).
+constexpr int kGapThreads = 1024;
+constexpr uint32_t kGapBlockBuckets = 1u << 15;
+__global__ void __launch_bounds__(kGapThreads) axisGapKernel(UnwrapAxes ax, uint32_t nb,
+                                                             const unsigned long long* __restrict__ bmin,
+                                                             const unsigned long long* __restrict__ bmax,
+                                                             unsigned long long* result /* {gap, anchor} per axis */,
+                                                             unsigned long long* suspect) {
+  __shared__ unsigned long long next_sm[2][kGapThreads];
+  __shared__ unsigned long long warp_max[kGapThreads / 32];
+  __shared__ unsigned long long best_sm;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const double box = pickAxis(ax.box, blockIdx.y);
+  bmin += static_cast<size_t>(blockIdx.y) * nb;
+  bmax += static_cast<size_t>(blockIdx.y) * nb;
+  const uint32_t per = (nb + kGapThreads - 1) / kGapThreads;
+  const uint32_t b0 = min(nb, t * per), b1 = min(nb, b0 + per);
+  unsigned long long first = ~0ull;
+  for (uint32_t b = b0; b < b1 && first == ~0ull; ++b) first = bmin[b];
+  // first value at or after this thread's buckets
+  int cur = 0;
+  next_sm[0][t] = first;
+  __syncthreads();
+  for (int off = 1; off < kGapThreads; off <<= 1) {
+    unsigned long long v = next_sm[cur][t];
+    if (v == ~0ull && t + off < kGapThreads) v = next_sm[cur][t + off];
+    next_sm[cur ^ 1][t] = v;
+    cur ^= 1;
+    __syncthreads();
+  }
+  const unsigned long long lowest = next_sm[cur][0];  // the smallest value of the axis
+  const unsigned long long after = t + 1 < kGapThreads ? next_sm[cur][t + 1] : ~0ull;
+  // pass 0: the largest gap; pass 1: the smallest value after a gap equal to it,
+  // and whether a bucket's own extent could hide one
+  unsigned long long best = 0ull, anchor = ~0ull, hidden = 0ull;
+  for (int pass = 0; pass < 2; ++pass) {
+    unsigned long long next = after;
+    for (uint32_t q = b1; q > b0; --q) {
+      const unsigned long long lo = bmin[q - 1];
+      if (lo == ~0ull) continue;
+      const double top = bitsd(bmax[q - 1]);
+      const bool around = next == ~0ull;
+      const unsigned long long to = around ? lowest : next;
+      const double cand = bitsd(to);
+      const double gap = (around ? cand + box : cand) - top;
+      if (pass == 0) {
+        best = dbits(gap) > best ? dbits(gap) : best;
+      } else {
+        if (dbits(gap) == best) anchor = to < anchor ? to : anchor;
+        if (lo != bmax[q - 1] && dbits(top - bitsd(lo)) >= best) hidden = 1ull;
+      }
+      next = lo;
+    }
+    if (pass == 0) {
+      for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
+        best = o > best ? o : best;
+      }
+      if (lane == 0) warp_max[warp] = best;
+      __syncthreads();
+      if (t == 0) {
+        unsigned long long v = 0ull;
+        for (int k = 0; k < kGapThreads / 32; ++k) v = warp_max[k] > v ? warp_max[k] : v;
+        best_sm = v;
+      }
+      __syncthreads();
+      best = best_sm;
+    }
+  }
+  if (anchor != ~0ull) atomicMin(result + 2 * blockIdx.y + 1, anchor);
+  if (hidden) atomicOr(suspect + blockIdx.y, 1ull);
+  if (t == 0) result[2 * blockIdx.y] = best;
 }
 
 // flag[k] = 1 for a non-empty bucket (flag[nb] = 0: the scan's total slot)
@@ -179,17 +282,38 @@ __global__ void __launch_bounds__(256) runGapKernel(int64_t m, const uint32_t* _
   }
 }
 
-// u += L below the anchor; skipped while the axis's bucket gaps are suspect.
-__global__ void applyAnchorKernel(int64_t n, double* u, double box, const unsigned long long* anchor_bits,
-                                  const unsigned long long* suspect) {
-  if (suspect && *suspect) return;
-  const double anchor = bitsd(*anchor_bits);
+// u += L below the anchor (not while the axis's bucket gaps are suspect), and the
+// bounds of the axis's unwrapped coordinates: bounds[axis] the smallest,
+// bounds[3 + axis] the largest, one axis per blockIdx.y.
+__global__ void __launch_bounds__(256) anchorBoundsKernel(int64_t n, UnwrapAxes ax, int first,
+                                                          const unsigned long long* __restrict__ result,
+                                                          const unsigned long long* __restrict__ suspect,
+                                                          unsigned long long* bounds) {
+  const int k = first + static_cast<int>(blockIdx.y);
+  if (suspect && suspect[k]) return;
+  double* __restrict__ u = pickAxis(ax.out, k);
+  const double box = pickAxis(ax.box, k);
+  const double anchor = bitsd(result[2 * k + 1]);
+  double lo = INFINITY, hi = -INFINITY;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (u[i] < anchor) u[i] += box;
+    double v = u[i];
+    if (v < anchor) {
+      v += box;
+      u[i] = v;
+    }
+    lo = fmin(lo, v);
+    hi = fmax(hi, v);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(bounds + k, orderedBits(lo));
+    atomicMax(bounds + 3 + k, orderedBits(hi));
   }
 }
-
 
 // ------------------------------------------------------------- bounds
 
@@ -266,7 +390,8 @@ __global__ void mortonKernel(int64_t n, const double* __restrict__ ux, const dou
 __global__ void pathKernel(int64_t n, int words, const uint32_t* __restrict__ perm,
                            const double* __restrict__ ux, const double* __restrict__ uy,
                            const double* __restrict__ uz, double cx0, double cy0, double cz0,
-                           double half0, unsigned long long mask0, unsigned long long* path /* words * n */) {
+                           double half0, unsigned long long mask0, unsigned long long* path /* words * n */,
+                           uint32_t* rows) {
   for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < n;
        j += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const uint32_t p = perm ? perm[j] : static_cast<uint32_t>(j);
@@ -285,6 +410,7 @@ __global__ void pathKernel(int64_t n, int words, const uint32_t* __restrict__ pe
       }
       path[static_cast<size_t>(w) * n + j] = w == 0 ? word & mask0 : word;
     }
+    rows[j] = static_cast<uint32_t>(j);
   }
 }
 
@@ -772,9 +898,14 @@ __global__ void momentsKernel(int64_t nodes, MomentIn in, const double4* __restr
 }
 
 // FP32 COM offset from the node centre and |centre - COM| for the walk's
-// single-precision acceptance tests.
-__global__ void nodeFrameKernel(int64_t nodes, const double4* __restrict__ geom, const double4* __restrict__ com,
-                                const double* __restrict__ quad, float4* f4, float4* mq) {
+// single-precision acceptance tests; in the same pass the bounds of the node
+// centres and COMs (the exact decisions' metric) and the largest depth.
+__global__ void __launch_bounds__(256) nodeFrameKernel(int64_t nodes, const double4* __restrict__ geom,
+                                                       const double4* __restrict__ com, const double* __restrict__ quad,
+                                                       const uint32_t* __restrict__ depth, float4* f4, float4* mq,
+                                                       unsigned long long* bounds /* 6, then the largest depth */) {
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  unsigned long long deepest = 0ull;
   for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < nodes;
        k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const double4 g = geom[k], c = com[k];
@@ -787,32 +918,32 @@ __global__ void nodeFrameKernel(int64_t nodes, const double4* __restrict__ geom,
                             static_cast<float>(q[1] / 3.0), static_cast<float>(q[2] / 3.0));
     mq[2 * k + 1] = make_float4(static_cast<float>((q[3] + tr) / 3.0), static_cast<float>(q[4] / 3.0),
                                 static_cast<float>((q[5] + tr) / 3.0), static_cast<float>(tr));
-  }
-}
-
-__global__ void nodeBoundsKernel(int64_t nodes, const double4* __restrict__ geom,
-                                 const double4* __restrict__ com, unsigned long long* out) {
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < nodes;
-       k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const double4 g = geom[k], c = com[k];
-    const double a[3] = {g.x, g.y, g.z}, b[3] = {c.x, c.y, c.z};
+    const double p[3] = {g.x, g.y, g.z}, b[3] = {c.x, c.y, c.z};
     for (int t = 0; t < 3; ++t) {
-      lo[t] = fmin(lo[t], fmin(a[t], b[t]));
-      hi[t] = fmax(hi[t], fmax(a[t], b[t]));
+      lo[t] = fmin(lo[t], fmin(p[t], b[t]));
+      hi[t] = fmax(hi[t], fmax(p[t], b[t]));
     }
+    deepest = depth[k] > deepest ? depth[k] : deepest;
   }
-  for (int a = 0; a < 3; ++a) {
+  // per block, then one set of atomics
+  __shared__ double part[7][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[7] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], static_cast<double>(deepest)};
+  for (int t = 0; t < 7; ++t) {
     for (int off = 16; off > 0; off >>= 1) {
-      lo[a] = fmin(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-      hi[a] = fmax(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+      const double o = __shfl_xor_sync(0xffffffffu, v[t], off);
+      v[t] = t < 3 ? fmin(v[t], o) : fmax(v[t], o);
     }
+    if (lane == 0) part[t][warp] = v[t];
   }
-  if ((threadIdx.x & 31) == 0) {
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(out + a, orderedBits(lo[a]));
-      atomicMax(out + 3 + a, orderedBits(hi[a]));
-    }
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    const int t = threadIdx.x;
+    double r = part[t][0];
+    for (int k = 1; k < 8; ++k) r = t < 3 ? fmin(r, part[t][k]) : fmax(r, part[t][k]);
+    if (t < 3) atomicMin(bounds + t, orderedBits(r));
+    else if (t < 6) atomicMax(bounds + t, orderedBits(r));
+    else atomicMax(bounds + 6, static_cast<unsigned long long>(r));
   }
 }
 
@@ -881,7 +1012,8 @@ int bitsFor(uint64_t maxval) {
 #define CHUI_GAP_BUCKET_DIV 8  // about n / 8 gap buckets per axis (n / 4: 9.3 ms tree build at 256^3, n / 8: 8.8)
 #endif
 
-// Unwrap the axes into `out` (tree frame), returning each axis's anchor. Per
+// Unwrap the axes into `out` (tree frame), returning each axis's anchor and the
+// bounds of its unwrapped coordinates. Per
 // axis, the canonical coordinates go into about n/8 gap buckets (min and max
 // per bucket), the non-empty buckets are listed in order, and the largest
 // circular gap is taken between consecutive buckets. When every bucket's own
@@ -891,55 +1023,75 @@ int bitsFor(uint64_t maxval) {
 // coordinates are sorted and the gaps taken between consecutive values, as
 // the reference does.
 static int unwrapAxes(Context& c, int64_t n, int axes, const int* axis, const double* const* in, const double* box,
-                      const int* canonical, double* const* out, double* anchor, cudaStream_t s) {
+                      const int* canonical, double* const* out, double* anchor, double* lo, double* hi, cudaStream_t s) {
   if (n == 0 || axes == 0) {
     for (int k = 0; k < axes; ++k) anchor[axis[k]] = 0.0;
     return 0;
   }
   uint32_t nb = 1;
   while (nb < static_cast<uint64_t>(n) / CHUI_GAP_BUCKET_DIV && nb < (1u << 30)) nb <<= 1;
-  if (ensure(c.bucket_min, static_cast<size_t>(nb) * 8) || ensure(c.bucket_max, static_cast<size_t>(nb) * 8) ||
-      ensure(c.gap_min, static_cast<size_t>(nb) * 8) || ensure(c.gap_max, static_cast<size_t>(nb) * 8) ||
-      ensure(c.gap_flag, (static_cast<size_t>(nb) + 1) * 4) || ensure(c.gap_off, (static_cast<size_t>(nb) + 1) * 4))
+  const bool one_block = nb <= kGapBlockBuckets;  // all axes at once, gaps by one block per axis
+  const size_t sets = one_block ? static_cast<size_t>(axes) : 1;
+  if (ensure(c.bucket_min, sets * nb * 8) || ensure(c.bucket_max, sets * nb * 8)) return CHUI_TREEPM_ENOMEM;
+  if (!one_block &&
+      (ensure(c.gap_min, static_cast<size_t>(nb) * 8) || ensure(c.gap_max, static_cast<size_t>(nb) * 8) ||
+       ensure(c.gap_flag, (static_cast<size_t>(nb) + 1) * 4) || ensure(c.gap_off, (static_cast<size_t>(nb) + 1) * 4)))
     return CHUI_TREEPM_ENOMEM;
+  // scalars: {gap, anchor} per axis slot, suspect flags at 6, bounds at 9 (by slot)
   auto* sc = c.scalars.as<unsigned long long>();
-  unsigned long long* suspect = sc + 16;  // one flag per axis slot
-  unsigned long long init[6] = {0ull, ~0ull, 0ull, ~0ull, 0ull, ~0ull};
+  unsigned long long* suspect = sc + 6;
+  unsigned long long* bounds = sc + 9;
+  const unsigned long long init[15] = {0ull, ~0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull, 0ull, 0ull,
+                                       ~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
   cudaMemcpyAsync(sc, init, sizeof(init), cudaMemcpyHostToDevice, s);
-  cudaMemsetAsync(suspect, 0, 3 * 8, s);
   unsigned long long* bmin = c.bucket_min.as<unsigned long long>();
   unsigned long long* bmax = c.bucket_max.as<unsigned long long>();
-  uint32_t* flag = c.gap_flag.as<uint32_t>();
-  uint32_t* off = c.gap_off.as<uint32_t>();
+  UnwrapAxes ua{};
   for (int k = 0; k < axes; ++k) {
     const int a = axis[k];
-    unsigned long long* g = sc + 2 * k;
-    cudaMemsetAsync(bmin, 0xFF, static_cast<size_t>(nb) * 8, s);
-    cudaMemsetAsync(bmax, 0, static_cast<size_t>(nb) * 8, s);
-    const double scale = static_cast<double>(nb) / box[a];
-    { noteLaunch(); canonicalBucketsKernel<<<gridFor(n, 256), 256, 0, s>>>(n, in[a], box[a], canonical[a], out[a], scale,
-                                                                       nb, bmin, bmax); }
-    { noteLaunch(); bucketFlagsKernel<<<gridFor(static_cast<size_t>(nb) + 1, 256), 256, 0, s>>>(nb, bmin, flag); }
-    if (int rc = exclusiveScanU32(c, flag, off, static_cast<int64_t>(nb) + 1, s)) return rc;
-    { noteLaunch(); bucketCompactKernel<<<gridFor(nb, 256), 256, 0, s>>>(nb, bmin, bmax, off, c.gap_min.as<unsigned long long>(),
-                                                                     c.gap_max.as<unsigned long long>()); }
-    for (int pass = 0; pass < 2; ++pass) {
-      noteLaunch();
-      runGapKernel<<<gridFor(nb, 256), 256, 0, s>>>(nb, off + nb, c.gap_min.as<unsigned long long>(),
-                                                    c.gap_max.as<unsigned long long>(), box[a], g, pass, g + 1,
-                                                    suspect + k);
-    }
-    { noteLaunch(); applyAnchorKernel<<<gridFor(n, 256), 256, 0, s>>>(n, out[a], box[a], g + 1, suspect + k); }
+    ua.in[k] = in[a];
+    ua.out[k] = out[a];
+    ua.box[k] = box[a];
+    ua.scale[k] = static_cast<double>(nb) / box[a];
+    ua.canonical[k] = canonical[a];
   }
-  unsigned long long ab[6], sus[3];
-  cudaMemcpyAsync(ab, sc, sizeof(ab), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(sus, suspect, sizeof(sus), cudaMemcpyDeviceToHost, s);
+  const unsigned ny = static_cast<unsigned>(axes);
+  if (one_block) {
+    cudaMemsetAsync(bmin, 0xFF, sets * nb * 8, s);
+    cudaMemsetAsync(bmax, 0, sets * nb * 8, s);
+    { noteLaunch(); canonicalBucketsKernel<<<dim3(gridFor(n, 256), ny), 256, 0, s>>>(n, ua, 0, nb, bmin, bmax); }
+    { noteLaunch(); axisGapKernel<<<dim3(1, ny), kGapThreads, 0, s>>>(ua, nb, bmin, bmax, sc, suspect); }
+  } else {
+    uint32_t* flag = c.gap_flag.as<uint32_t>();
+    uint32_t* off = c.gap_off.as<uint32_t>();
+    for (int k = 0; k < axes; ++k) {
+      unsigned long long* g = sc + 2 * k;
+      cudaMemsetAsync(bmin, 0xFF, static_cast<size_t>(nb) * 8, s);
+      cudaMemsetAsync(bmax, 0, static_cast<size_t>(nb) * 8, s);
+      { noteLaunch(); canonicalBucketsKernel<<<gridFor(n, 256), 256, 0, s>>>(n, ua, k, nb, bmin, bmax); }
+      { noteLaunch(); bucketFlagsKernel<<<gridFor(static_cast<size_t>(nb) + 1, 256), 256, 0, s>>>(nb, bmin, flag); }
+      if (int rc = exclusiveScanU32(c, flag, off, static_cast<int64_t>(nb) + 1, s)) return rc;
+      { noteLaunch(); bucketCompactKernel<<<gridFor(nb, 256), 256, 0, s>>>(nb, bmin, bmax, off, c.gap_min.as<unsigned long long>(),
+                                                                       c.gap_max.as<unsigned long long>()); }
+      for (int pass = 0; pass < 2; ++pass) {
+        noteLaunch();
+        runGapKernel<<<gridFor(nb, 256), 256, 0, s>>>(nb, off + nb, c.gap_min.as<unsigned long long>(),
+                                                      c.gap_max.as<unsigned long long>(), ua.box[k], g, pass, g + 1,
+                                                      suspect + k);
+      }
+    }
+  }
+  const unsigned reduce_blocks = std::min(gridFor(n, 256), kReduceBlocks);
+  { noteLaunch(); anchorBoundsKernel<<<dim3(reduce_blocks, ny), 256, 0, s>>>(n, ua, 0, sc, suspect, bounds); }
+  unsigned long long* got = c.pinned;
+  cudaMemcpyAsync(got, sc, 15 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
-  bool resorted = false;
+  c.unwrap_sorted_axes = 0;
   for (int k = 0; k < axes; ++k) {
-    if (!sus[k]) continue;
+    if (!got[6 + k]) continue;
     // out[a] still holds the canonical coordinates (the anchor was skipped)
     const int a = axis[k];
+    c.unwrap_sorted_axes |= 1 << a;
     if (ensure(c.keys_b, static_cast<size_t>(n) * 8)) return CHUI_TREEPM_ENOMEM;
     const unsigned long long* kin = reinterpret_cast<const unsigned long long*>(out[a]);
     unsigned long long* sorted = c.keys_b.as<unsigned long long>();
@@ -952,15 +1104,16 @@ static int unwrapAxes(Context& c, int64_t n, int axes, const int* axis, const do
       noteLaunch();
       runGapKernel<<<gridFor(n, 256), 256, 0, s>>>(n, nullptr, sorted, sorted, box[a], g, pass, g + 1, nullptr);
     }
-    { noteLaunch(); applyAnchorKernel<<<gridFor(n, 256), 256, 0, s>>>(n, out[a], box[a], g + 1, nullptr); }
-    cudaMemcpyAsync(&ab[2 * k], g, 16, cudaMemcpyDeviceToHost, s);
-    resorted = true;
+    { noteLaunch(); anchorBoundsKernel<<<dim3(reduce_blocks, 1), 256, 0, s>>>(n, ua, k, sc, nullptr, bounds); }
   }
-  if (resorted && cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
-  c.unwrap_sorted_axes = 0;
+  if (c.unwrap_sorted_axes) {
+    cudaMemcpyAsync(got, sc, 15 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
+  }
   for (int k = 0; k < axes; ++k) {
-    std::memcpy(&anchor[axis[k]], &ab[2 * k + 1], 8);
-    if (sus[k]) c.unwrap_sorted_axes |= 1 << axis[k];
+    std::memcpy(&anchor[axis[k]], &got[2 * k + 1], 8);
+    lo[axis[k]] = fromOrderedBits(got[9 + k]);
+    hi[axis[k]] = fromOrderedBits(got[12 + k]);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : CHUI_TREEPM_EDEVICE;
 }
@@ -973,6 +1126,10 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
   c.unwrap_sorted_axes = 0;
   c.large_leaf = 0;
   c.path_levels_retried = 0;
+  for (int a = 0; a < 3; ++a) {
+    c.node_lo[a] = INFINITY;
+    c.node_hi[a] = -INFINITY;
+  }
   if (n == 0) return 0;
   const double box[3] = {c.cfg.box_x, c.cfg.box_y, c.cfg.box_z};
   if (ensure(c.ux, n * 8) || ensure(c.uy, n * 8) || ensure(c.uz, n * 8)) return CHUI_TREEPM_ENOMEM;
@@ -991,19 +1148,20 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
     }
     axis[axes++] = a;
   }
-  if (int rc = unwrapAxes(c, n, axes, axis, in, box, canonical, u, anchors, s)) return rc;
-  // bounds of the unwrapped frame
-  auto* sc = c.scalars.as<unsigned long long>();
-  unsigned long long init[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
-  cudaMemcpyAsync(sc, init, sizeof(init), cudaMemcpyHostToDevice, s);
-  { noteLaunch(); boundsKernel<<<std::min(gridFor(n, 256), kReduceBlocks), 256, 0, s>>>(n, u[0], u[1], u[2], sc); }
-  unsigned long long hb[6];
-  cudaMemcpyAsync(hb, sc, sizeof(hb), cudaMemcpyDeviceToHost, s);
-  cudaStreamSynchronize(s);
   double lo[3], hi[3];
-  for (int a = 0; a < 3; ++a) {
-    lo[a] = fromOrderedBits(hb[a]);
-    hi[a] = fromOrderedBits(hb[3 + a]);
+  if (int rc = unwrapAxes(c, n, axes, axis, in, box, canonical, u, anchors, lo, hi, s)) return rc;
+  if (axes == 0) {
+    // isolated/open: bounds of the caller's coordinates
+    auto* sc = c.scalars.as<unsigned long long>();
+    const unsigned long long init[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
+    cudaMemcpyAsync(sc, init, sizeof(init), cudaMemcpyHostToDevice, s);
+    { noteLaunch(); boundsKernel<<<std::min(gridFor(n, 256), kReduceBlocks), 256, 0, s>>>(n, u[0], u[1], u[2], sc); }
+    cudaMemcpyAsync(c.pinned, sc, sizeof(init), cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = fromOrderedBits(c.pinned[a]);
+      hi[a] = fromOrderedBits(c.pinned[3 + a]);
+    }
   }
   const double max_extent = std::fmax(hi[0] - lo[0], std::fmax(hi[1] - lo[1], hi[2] - lo[2]));
 
@@ -1074,10 +1232,9 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
     const int levels = masked ? masked_levels : kLevelsPerWord * words;
     const unsigned long long mask0 = masked ? ~((1ull << (3 * (kLevelsPerWord - masked_levels))) - 1ull) : ~0ull;
     { noteLaunch(); pathKernel<<<gridFor(n, 256), 256, 0, s>>>(n, words, nullptr, u[0], u[1], u[2], cx0, cy0, cz0, half0,
-                                               mask0, by_row); }
+                                               mask0, by_row, c.idx_c.as<uint32_t>()); }
     uint32_t* rank_in = c.idx_c.as<uint32_t>();
     uint32_t* rank_out = c.idx_d.as<uint32_t>();
-    { noteLaunch(); iotaKernel<<<gridFor(n, 256), 256, 0, s>>>(n, rank_in); }
     // LSD over path words, each pass a stable sort; the first pass reads the
     // words in row order and the last writes the sorted first word in place
     for (int w = words - 1; w >= 0; --w) {
@@ -1087,7 +1244,9 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
         gatherU64Kernel<<<gridFor(n, 256), 256, 0, s>>>(n, key_in, rank_in, key_cur);
         key_in = key_cur;
       }
-      rc = radixSortPairsU64(c, key_in, w == 0 ? path : key_sorted, rank_in, rank_out, n, 63, s);
+      // the zeroed low digits of a masked word are not sorted at all
+      rc = radixSortPairsU64(c, key_in, w == 0 ? path : key_sorted, rank_in, rank_out, n, 63, s,
+                             masked ? 3 * (kLevelsPerWord - masked_levels) : 0);
       if (rc) return rc;
       uint32_t* t = rank_in;
       rank_in = rank_out;
@@ -1103,7 +1262,7 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
     cudaMemsetAsync(status, 0, 4, s);
     { noteLaunch(); nodeCountKernel<<<gridFor(n + 1, 256), 256, 0, s>>>(plan, cp, counts, status); }
     if ((rc = exclusiveScanU32(c, counts, offset, n + 1, s))) return rc;
-    uint32_t hs[2];
+    uint32_t* hs = reinterpret_cast<uint32_t*>(c.pinned);
     cudaMemcpyAsync(&hs[0], status, 4, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(&hs[1], offset + n, 4, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
@@ -1178,9 +1337,9 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
                                                  chain_start, chain_off + n, lv, cx0, cy0, cz0, half0, total_nodes,
                                                  out, status); }
   {
-    uint32_t est = 0;
-    cudaMemcpyAsync(&est, status, 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(c.pinned, status, 4, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
+    const uint32_t est = *reinterpret_cast<uint32_t*>(c.pinned);
     if (est & ~static_cast<uint32_t>(kStatusLargeLeaf)) {
       c.last_error = "tree node enumeration produced an inconsistent node range";
       return CHUI_TREEPM_EDEVICE;
@@ -1242,46 +1401,37 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
                                                           c.node_com.as<double4>(), c.node_quad.as<double>()); }
   if (ensure(c.node_f4, total_nodes * sizeof(float4)) || ensure(c.node_mq, total_nodes * 2 * sizeof(float4)))
     return CHUI_TREEPM_ENOMEM;
-  { noteLaunch(); nodeFrameKernel<<<gridFor(total_nodes, 256), 256, 0, s>>>(total_nodes, out.geom, c.node_com.as<double4>(),
-                                                            c.node_quad.as<double>(), c.node_f4.as<float4>(),
-                                                            c.node_mq.as<float4>()); }
-  // maximum depth (for stack sizing and stats); the status of the
-  // within-leaf ordering is read at the same synchronisation
+  // node bounds (the walk's exact metric) and maximum depth (stack sizing and
+  // stats), read with the status of the within-leaf ordering
   {
-    uint32_t hd = 0, est = 0;
-    cudaMemcpyAsync(&est, status, 4, cudaMemcpyDeviceToHost, s);
-    if (maxU32(c, out.depth, total_nodes, &hd, s)) {
+    auto* sc = c.scalars.as<unsigned long long>();
+    const unsigned long long init[7] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull};
+    cudaMemcpyAsync(sc, init, sizeof(init), cudaMemcpyHostToDevice, s);
+    { noteLaunch(); nodeFrameKernel<<<std::min(gridFor(total_nodes, 256), kReduceBlocks), 256, 0, s>>>(
+        total_nodes, out.geom, c.node_com.as<double4>(), c.node_quad.as<double>(), out.depth, c.node_f4.as<float4>(),
+        c.node_mq.as<float4>(), sc); }
+    cudaMemcpyAsync(c.pinned, sc, sizeof(init), cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(c.pinned + 7, status, 4, cudaMemcpyDeviceToHost, s);
+    if (cudaStreamSynchronize(s) != cudaSuccess) {
       c.last_error = "tree build kernels failed";
       return CHUI_TREEPM_EDEVICE;
     }
+    const uint32_t est = *reinterpret_cast<uint32_t*>(c.pinned + 7);
     if (est & ~static_cast<uint32_t>(kStatusLargeLeaf)) {
       c.last_error = "tree leaf ordering produced an inconsistent index";
       return CHUI_TREEPM_EDEVICE;
     }
-    c.max_depth = hd;
-    c.prev_tree_depth = static_cast<int>(hd);
+    for (int a = 0; a < 3; ++a) {
+      c.node_lo[a] = fromOrderedBits(c.pinned[a]);
+      c.node_hi[a] = fromOrderedBits(c.pinned[3 + a]);
+    }
+    c.max_depth = static_cast<uint32_t>(c.pinned[6]);
+    c.prev_tree_depth = static_cast<int>(c.max_depth);
   }
   c.tree_anchor[0] = anchors[0];
   c.tree_anchor[1] = anchors[1];
   c.tree_anchor[2] = anchors[2];
   return cudaGetLastError() == cudaSuccess ? 0 : CHUI_TREEPM_EDEVICE;
-}
-
-int treeNodeBounds(Context& c, double lo[3], double hi[3], cudaStream_t s) {
-  auto* sc = c.scalars.as<unsigned long long>();
-  unsigned long long init[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
-  cudaMemcpyAsync(sc, init, sizeof(init), cudaMemcpyHostToDevice, s);
-  if (c.n_nodes > 0)
-    { noteLaunch(); nodeBoundsKernel<<<std::min(gridFor(c.n_nodes, 256), kReduceBlocks), 256, 0, s>>>(c.n_nodes, c.node_geom.as<double4>(),
-                                                              c.node_com.as<double4>(), sc); }
-  unsigned long long hb[6];
-  cudaMemcpyAsync(hb, sc, sizeof(hb), cudaMemcpyDeviceToHost, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) return CHUI_TREEPM_EDEVICE;
-  for (int a = 0; a < 3; ++a) {
-    lo[a] = c.n_nodes > 0 ? fromOrderedBits(hb[a]) : INFINITY;
-    hi[a] = c.n_nodes > 0 ? fromOrderedBits(hb[3 + a]) : -INFINITY;
-  }
-  return 0;
 }
 
 // Visit order: active slots sorted by the tree position of their row
