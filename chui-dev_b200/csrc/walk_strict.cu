@@ -103,8 +103,10 @@ __device__ __forceinline__ double callerOffset(double d, double near, double len
 // targets, at most `most` of them, whose extent stays within `limit` per axis
 // (a run that straddles a jump of the tree order would walk the tree with a
 // box that spans the jump). One warp per 32 positions.
-// A run whose targets spread beyond two r_cut but not beyond the reach of the
-// nearest image (r_cut + spread below half a box) is marked kWideRun.
+// A run whose targets spread beyond a quarter of r_cut, but not beyond the reach
+// of the nearest image (r_cut + spread below half a box), is marked kWideRun:
+// its groups keep the run's first target as the origin of their FP32 offsets,
+// so its closest pairs keep the rounding they have in a frame for the run.
 __global__ void __launch_bounds__(256) targetGroupsKernel(WalkArgs a, int most, double limit, uint2* groups,
                                                           uint32_t* count) {
   const int lane = threadIdx.x & 31;
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(256) targetGroupsKernel(WalkArgs a, int most, 
       const double sz = frameImage(pz - __shfl_sync(0xffffffffu, pz, 0), w.box[2], w.inv_box[2]);
       const double spread = fmax(fabs(sx), fmax(fabs(sy), fabs(sz)));
       const double nearest = w.box[0] > 0.0 ? 0.5 * fmin(w.box[0], fmin(w.box[1], w.box[2])) : INFINITY;
-      const bool far = __any_sync(0xffffffffu, valid && spread > 2.0 * w.cutoff);
+      const bool far = __any_sync(0xffffffffu, valid && spread > 0.25 * w.cutoff);
       const bool ambiguous = __any_sync(0xffffffffu, valid && w.cutoff + spread >= nearest);
       if (far && !ambiguous) wide = kWideRun;
     }
@@ -406,8 +408,8 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
 
     // Queue the sources [begin, begin + count) within r_cut of the box, as
     // offsets from (sx, sy, sz): the box centre moved to the sources' image.
-    // `lanes` take them.
-    auto enqueue = [&](uint32_t begin, uint32_t count, uint32_t lanes, double sx, double sy, double sz) {
+    // `lanes` take them; `inside`: every one is within r_cut of every target.
+    auto enqueue = [&](uint32_t begin, uint32_t count, uint32_t lanes, bool inside, double sx, double sy, double sz) {
       const double4* src = a.src_u4 + begin;
       // rounding of the box's position in the frame
       const float slack = 2.4e-7f * fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz)));
@@ -433,9 +435,12 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
           }
         }
         const float ex = static_cast<float>(dx), ey = static_cast<float>(dy), ez = static_cast<float>(dz);
-        const float gx = fmaxf(fabsf(ex - bx) - (hbx + slack), 0.f), gy = fmaxf(fabsf(ey - by) - (hby + slack), 0.f),
-                    gz = fmaxf(fabsf(ez - bz) - (hbz + slack), 0.f);
-        const bool keep = have && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= cut_hi2;
+        bool keep = have;
+        if (!inside) {
+          const float gx = fmaxf(fabsf(ex - bx) - (hbx + slack), 0.f), gy = fmaxf(fabsf(ey - by) - (hby + slack), 0.f),
+                      gz = fmaxf(fabsf(ez - bz) - (hbz + slack), 0.f);
+          keep = have && fmaf(gx, gx, fmaf(gy, gy, gz * gz)) <= cut_hi2;
+        }
         const uint32_t kept = __ballot_sync(0xffffffffu, keep);
         if (keep) {
           const int o = qn + __popc(kept & ((1u << lane) - 1u));
@@ -632,6 +637,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
                                    (Lz > 0.f && r.az + hbz + rc >= Lz * 0.99999f));
       const unsigned moved = __ballot_sync(0xffffffffu, emit && (r.kx != 0.0 || r.ky != 0.0 || r.kz != 0.0));
       const unsigned many = __ballot_sync(0xffffffffu, images);
+      const unsigned within = __ballot_sync(0xffffffffu, r.far2 <= cut_lo2);  // no source to cull
       for (unsigned todo = __ballot_sync(0xffffffffu, emit); todo; todo &= todo - 1u) {
         const int j = __ffs(todo) - 1;
         const uint32_t begin = __shfl_sync(0xffffffffu, rg.x, j), count = __shfl_sync(0xffffffffu, rg.y, j);
@@ -656,7 +662,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
             continue;
           // the nearest image of a node around the group keeps the origin's bits
           // (a target's own entry stays at distance zero)
-          enqueue(begin, count, lanes, fx0 + w.box[0] * (jx - ix), fy0 + w.box[1] * (jy - iy), fz0 + w.box[2] * (jz - iz));
+          enqueue(begin, count, lanes, !each && ((within >> j) & 1u) != 0u, fx0 + w.box[0] * (jx - ix), fy0 + w.box[1] * (jy - iy), fz0 + w.box[2] * (jz - iz));
         }
       }
     }
