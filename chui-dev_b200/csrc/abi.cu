@@ -37,7 +37,49 @@ void release(DevBuf& b) {
 
 namespace {
 std::atomic<uint64_t> g_launches{0};
+
+// Page-locked result words of the contexts: 32 slots of 16 words in one 4 KiB
+// page of the process (page-locking takes up to a millisecond, as much as a
+// small solve), taken at creation and given back at destruction; the page goes
+// with its last user. Contexts beyond 32 lock their own.
+constexpr int kPinnedSlots = 32, kPinnedWords = 16;
+std::mutex g_pinned_lock;
+unsigned long long* g_pinned_page = nullptr;
+uint32_t g_pinned_used = 0;
+
+unsigned long long* lockedWords(int words) {
+  void* p = nullptr;
+  return cudaHostAlloc(&p, static_cast<size_t>(words) * 8, cudaHostAllocPortable) == cudaSuccess
+             ? static_cast<unsigned long long*>(p)
+             : nullptr;
 }
+
+unsigned long long* takePinned() {
+  std::lock_guard<std::mutex> hold(g_pinned_lock);
+  if (!g_pinned_page) g_pinned_page = lockedWords(kPinnedSlots * kPinnedWords);
+  if (!g_pinned_page) return nullptr;
+  for (int k = 0; k < kPinnedSlots; ++k) {
+    if (g_pinned_used & (1u << k)) continue;
+    g_pinned_used |= 1u << k;
+    return g_pinned_page + k * kPinnedWords;
+  }
+  return lockedWords(kPinnedWords);
+}
+
+void givePinned(unsigned long long* p) {
+  if (!p) return;
+  std::lock_guard<std::mutex> hold(g_pinned_lock);
+  if (!g_pinned_page || p < g_pinned_page || p >= g_pinned_page + kPinnedSlots * kPinnedWords) {
+    cudaFreeHost(p);
+    return;
+  }
+  g_pinned_used &= ~(1u << ((p - g_pinned_page) / kPinnedWords));
+  if (g_pinned_used == 0) {
+    cudaFreeHost(g_pinned_page);
+    g_pinned_page = nullptr;
+  }
+}
+}  // namespace
 void noteLaunch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 uint64_t launchCount() { return g_launches.load(std::memory_order_relaxed); }
 
@@ -792,7 +834,7 @@ int chui_treepm_create(const chui_treepm_config* cfg, void** handle) {
   chui::DeviceGuard guard(c->device);
   chui::applyConfig(*c, *cfg);
   if (chui::ensure(c->status, 64) != cudaSuccess || chui::ensure(c->scalars, 64 * 8) != cudaSuccess ||
-      cudaHostAlloc(reinterpret_cast<void**>(&c->pinned), 16 * 8, cudaHostAllocDefault) != cudaSuccess) {
+      (c->pinned = chui::takePinned()) == nullptr) {
     chui::release(c->status);
     chui::release(c->scalars);
     delete c;
@@ -828,7 +870,7 @@ void chui_treepm_destroy(void* handle) {
                             &c->tree_acc, &c->tree_near, &c->walk_cost, &c->walk_groups, &c->out_lr[0], &c->out_lr[1],
                             &c->out_lr[2]};
     for (auto* b : bufs) chui::release(*b);
-    cudaFreeHost(c->pinned);
+    chui::givePinned(c->pinned);
     if (c->events_ready)
       for (auto& e : c->ev) cudaEventDestroy(e);
     if (c->pipe_ready) {
@@ -1056,6 +1098,10 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
     return chui::fail(c, CHUI_TREEPM_ESTATE, "TreePM long-range reuse requested without a compatible PM field");
   }
 
+  // the production walk also counts and records nearest pairs when asked to,
+  // or when the caller wants the nearest-pair lane
+  c.walk_instrument = c.cfg.diagnostics == 2 || acc->nearest_pair_r2 != nullptr;
+  c.leaf_offsets = c.cfg.acceptance_policy != CHUI_TREEPM_POLICY_STRICT || c.cfg.diagnostics == 1 || c.walk_instrument;
   // periodic tree build (first: the PM deposit reads the tree-ordered sources);
   // equal masses travel as one value instead of a lane of scattered reads
   const bool equal_masses = m && mass_range[0] == mass_range[1];
@@ -1127,9 +1173,6 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
   wp.eps2_f = static_cast<float>(c.cfg.softening * c.cfg.softening);
   wp.G_f = static_cast<float>(c.cfg.gravitational_constant);
   cudaMemsetAsync(c.status.ptr, 0, 4, s);
-  // the production walk also counts and records nearest pairs when asked to,
-  // or when the caller wants the nearest-pair lane
-  c.walk_instrument = c.cfg.diagnostics == 2 || acc->nearest_pair_r2 != nullptr;
   // outputs at slots (a slice's compactly, with per-block cycles)
   if (n > 0 && (rc = chui::walkRun(c, nt, active, tx, ty, tz, x, y, z, prev, wp, n, s, visit_begin, visit_end,
                                      ranged, ranged)))
@@ -1393,6 +1436,7 @@ int chui_treepm_force_vjp(void* handle, const chui_treepm_sources* src, const do
     gy = c.out_acc[1].as<double>();
     gz = c.out_acc[2].as<double>();
   }
+  c.leaf_offsets = false;
   // tree for these positions, every particle a target in tree order
   c.visit_count = -1;
   if (n > 0) {

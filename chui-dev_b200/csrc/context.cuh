@@ -156,7 +156,8 @@ struct Context {
   DevBuf node_counter; // u32 (bottom-up completion counters)
   DevBuf sorted_index; // u32 per tree position: caller row
   DevBuf pos_of_row;   // u32 per caller row: tree position
-  DevBuf src_f4;       // float4 per tree position: offset from leaf centre (FP32) + mass
+  DevBuf src_f4;       // float4 per tree position: offset from leaf centre (FP32) + mass (leaf_offsets)
+  bool leaf_offsets = false;  // the current solve's walk reads src_f4 (adaptive and counting walks)
   DevBuf src_d4;       // double4 per tree position: caller position + mass (FP64 path)
   DevBuf src_u4;       // double4 per tree position: unwrapped (tree frame) position + mass (moments, walk)
   DevBuf src_cot;      // double4 per tree position: force cotangent (adjoint walk)

@@ -968,8 +968,8 @@ __global__ void scatterSourcesKernel(int64_t n, const uint32_t* __restrict__ pos
   }
 }
 
-// Mixed precision: each source's FP32 offset from its leaf's FP64 centre, in
-// tree order (a leaf's sources are consecutive).
+// Mixed precision, adaptive and counting walks: each source's FP32 offset from its
+// leaf's FP64 centre, in tree order (a leaf's sources are consecutive).
 __global__ void leafOffsetsKernel(int64_t n, const uint32_t* __restrict__ leaf_of_pos,
                                   const double4* __restrict__ geom, const double4* __restrict__ u4, float4* f4) {
   for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n;
@@ -1372,7 +1372,7 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
     if (rc) return rc;
   }
   // tree-ordered source records
-  const bool mixed = c.cfg.precision == CHUI_TREEPM_MIXED;
+  const bool mixed = c.cfg.precision == CHUI_TREEPM_MIXED && c.leaf_offsets;
   if (mixed) {
     if (ensure(c.src_f4, n * sizeof(float4))) return CHUI_TREEPM_ENOMEM;
   }

@@ -590,9 +590,6 @@ constexpr int kMultList = 4; // accepted multipoles per lane before a flush (4 a
 #ifndef CHUI_PAIR_UNROLL
 #define CHUI_PAIR_UNROLL 4  // source pairs per unrolled step of the pair loop
 #endif
-#ifndef CHUI_WALK_MIN_BLOCKS_STRICT
-#define CHUI_WALK_MIN_BLOCKS_STRICT 6  // the strict, uniform-mass production instances (80 registers)
-#endif
 #ifndef CHUI_WALK_MIN_BLOCKS
 #define CHUI_WALK_MIN_BLOCKS 5  // resident blocks per SM the register budget is sized for
 #endif
@@ -692,9 +689,7 @@ __device__ __forceinline__ void targetBox(bool valid, float off, float& c, float
 template <bool kEpsZero, int kTerms, bool kDiag, bool kContiguous, int kMode, bool kUniform = false,
           bool kCost = false, bool kF64 = false, bool kSoft = false>
 __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
-                                  (kMode == 0 && kUniform)   ? CHUI_WALK_MIN_BLOCKS_STRICT
-                                  : (kMode == 2 && kUniform) ? CHUI_WALK_MIN_BLOCKS_ADAPTIVE
-                                                             : CHUI_WALK_MIN_BLOCKS)
+                                  (kMode == 2 && kUniform) ? CHUI_WALK_MIN_BLOCKS_ADAPTIVE : CHUI_WALK_MIN_BLOCKS)
     walkFastKernel(WalkArgs a) {
   static_assert(!kF64 || (kMode <= 1 && !kDiag && !kUniform), "FP64 production walk: strict policy only");
   static_assert(!kSoft || (!kUniform && !kEpsZero && !kF64 && kMode <= 2), "per-particle softening instances");
