@@ -20,9 +20,9 @@
 //    region).
 //  - The pair loop reads four queued sources at a time from x, y, z arrays in
 //    shared memory and evaluates them two by two in packed FP32.
-// Bound by the FMA pipe of the pair loop (76 % of the walk at 256^3 clustered:
+// Bound by the FMA pipe of the pair loop (78 % of the walk at 256^3 clustered:
 // 2552 quads of sources per 32 targets at 54 ns per quad and scheduler is 122 of
-// 161 ms). Before, with one warp per 32 consecutive targets whatever their spread,
+// 156 ms). Before, with one warp per 32 consecutive targets whatever their spread,
 // every node decided per lane and sources culled by a sphere: 193 ms at 256^3,
 // 33 to 46 ms against 15.6 at 128^3, 20 against 1.8 ms for 200 k particles (a
 // warp straddling a jump of the tree order walked for milliseconds).
