@@ -135,6 +135,7 @@ struct Context {
   uint32_t max_depth = 0;
   double root_half = 0.0;  // half-size of the root node
   double node_lo[3] = {}, node_hi[3] = {};  // bounds of node centres and COMs
+  double frame_lo[3] = {}, frame_hi[3] = {};  // bounds of the sources in the tree frame
   unsigned long long* pinned = nullptr;     // 16 words of page-locked host memory for small results
   int path_words_used = 0;
   int unwrap_sorted_axes = 0;  // axes whose unwrap sorted the coordinates (bit a)

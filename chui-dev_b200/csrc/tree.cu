@@ -1163,6 +1163,10 @@ int treeBuild(Context& c, int64_t n, const double* x, const double* y, const dou
       hi[a] = fromOrderedBits(c.pinned[3 + a]);
     }
   }
+  for (int a = 0; a < 3; ++a) {
+    c.frame_lo[a] = lo[a];
+    c.frame_hi[a] = hi[a];
+  }
   const double max_extent = std::fmax(hi[0] - lo[0], std::fmax(hi[1] - lo[1], hi[2] - lo[2]));
 
   // Morton keys (tree_ordering.cpp:152-172). The reference sorts them and

@@ -85,6 +85,11 @@ struct WalkArgs {
   WalkParams wp;
 };
 
+// Bounds of the sources in the tree frame.
+struct SourceFrame {
+  double lo[3], hi[3];
+};
+
 // The strict production walk's own arguments (walk_strict.cu).
 struct StrictArgs {
   int targets_per_group;        // at most; a power of two
@@ -96,6 +101,7 @@ struct StrictArgs {
   double h64[kPoly64Max];       // FP64: H(t)/(8 r_s^3) in s = r^2 h64_scale - 1
   double h64_scale;
   int caller_sources;           // FP64: sources at the caller's coordinates instead of the tree frame's
+  SourceFrame frame;
 };
 
 namespace {
@@ -522,6 +528,24 @@ __device__ __forceinline__ NodeReach nodeReach(const double4* __restrict__ geom,
   return r;
 }
 
+// One axis of the images of a node that some target may reach: its sources lie
+// in the part of its cube (centre nd from the image k of the box centre c,
+// half-size h) inside the bounds of all sources, and come within r_cut of the
+// targets' box (half extent hb) when moved back by k, k + 1, ... k + count - 1
+// box lengths. The cube of a sparse leaf can span several short sides of an
+// elongated box, its centre lengths away from its sources, so the images are
+// counted from the sources' interval (three at most: it is no wider than L, and
+// r_cut + hb stays below 0.63 L).
+__device__ __forceinline__ void nodeImages(const WalkParams& w, const SourceFrame& s, int axis, double nd, double h,
+                                           double c, double hb, double& k, int& count) {
+  const double L = w.box[axis];
+  if (!(L > 0.0)) return;
+  const double centre = nd + L * k, reach = w.cutoff + hb + 1.0e-5 * L;  // with room for rounding
+  const double lo = fmax(centre - h, s.lo[axis] - c) - reach, hi = fmin(centre + h, s.hi[axis] - c) + reach;
+  k = ceil(lo * w.inv_box[axis]);
+  count = 1 + static_cast<int>(fmin(fmax(floor(hi * w.inv_box[axis]) - k, 0.0), 3.0));
+}
+
 // The children of the lanes' nodes that are opened (push) go on the stack, each
 // with `flag` set; returns the new height, or sets overflow.
 __device__ __forceinline__ int pushChildren(const uint32_t* __restrict__ child, uint32_t node, bool push,
@@ -555,6 +579,15 @@ __device__ __forceinline__ int pushChildren(const uint32_t* __restrict__ child, 
   }
   __syncwarp();
   return sp + static_cast<int>(total);
+}
+
+inline SourceFrame sourceFrame(const Context& c) {
+  SourceFrame f;
+  for (int a = 0; a < 3; ++a) {
+    f.lo[a] = c.frame_lo[a];
+    f.hi[a] = c.frame_hi[a];
+  }
+  return f;
 }
 
 }  // namespace

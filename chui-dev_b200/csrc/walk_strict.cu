@@ -34,8 +34,8 @@
 //
 // Periodic images: a node is placed at its nearest image of the box centre, and
 // where the reach of the group (box + r_cut + node) spans more than one image
-// its sources are queued once per image; a pair is inside r_cut < L/2 in one
-// image at most.
+// its sources are queued once per image that brings some of them into reach
+// (nodeImages); a pair is inside r_cut < L/2 in one image at most.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -643,26 +643,31 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
         const uint32_t begin = __shfl_sync(0xffffffffu, rg.x, j), count = __shfl_sync(0xffffffffu, rg.y, j);
         const uint32_t lanes = __shfl_sync(0xffffffffu, mask, j);
         const bool shift = ((moved >> j) & 1u) != 0u, each = ((many >> j) & 1u) != 0u;
-        double jx = 0.0, jy = 0.0, jz = 0.0, ox = 0.0, oy = 0.0, oz = 0.0, rr = 0.0;
+        double jx = 0.0, jy = 0.0, jz = 0.0;
+        int nx = 1, ny = 1, nz = 1;
         if (shift || each) {
           jx = __shfl_sync(0xffffffffu, r.kx, j);
           jy = __shfl_sync(0xffffffffu, r.ky, j);
           jz = __shfl_sync(0xffffffffu, r.kz, j);
         }
         if (each) {
-          ox = __shfl_sync(0xffffffffu, r.ndx, j);
-          oy = __shfl_sync(0xffffffffu, r.ndy, j);
-          oz = __shfl_sync(0xffffffffu, r.ndz, j);
-          rr = static_cast<double>(__shfl_sync(0xffffffffu, rc, j)) * 1.00001;
+          const double h = __shfl_sync(0xffffffffu, r.half, j);
+          nodeImages(w, sa.frame, 0, __shfl_sync(0xffffffffu, r.ndx, j), h, cx, hbx, jx, nx);
+          nodeImages(w, sa.frame, 1, __shfl_sync(0xffffffffu, r.ndy, j), h, cy, hby, jy, ny);
+          nodeImages(w, sa.frame, 2, __shfl_sync(0xffffffffu, r.ndz, j), h, cz, hbz, jz, nz);
         }
-        for (int im = each ? 0 : 13; im < (each ? 27 : 14); ++im) {
-          const int ix = im / 9 - 1, iy = im / 3 % 3 - 1, iz = im % 3 - 1;
-          if (each && (fabs(ox + ix * w.box[0]) > rr + hbx || fabs(oy + iy * w.box[1]) > rr + hby ||
-                       fabs(oz + iz * w.box[2]) > rr + hbz))
-            continue;
-          // the nearest image of a node around the group keeps the origin's bits
-          // (a target's own entry stays at distance zero)
-          enqueue(begin, count, lanes, !each && ((within >> j) & 1u) != 0u, fx0 + w.box[0] * (jx - ix), fy0 + w.box[1] * (jy - iy), fz0 + w.box[2] * (jz - iz));
+        for (int ix = 0, iy = 0, iz = 0; iz < nz;) {
+          // unmoved sources keep the origin's bits (a target's own entry stays at
+          // distance zero)
+          enqueue(begin, count, lanes, !each && ((within >> j) & 1u) != 0u, fx0 + w.box[0] * (jx + ix),
+                  fy0 + w.box[1] * (jy + iy), fz0 + w.box[2] * (jz + iz));
+          if (++ix == nx) {
+            ix = 0;
+            if (++iy == ny) {
+              iy = 0;
+              ++iz;
+            }
+          }
         }
       }
     }
@@ -751,6 +756,7 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
   const bool blocks = !tiny || !a.wp.quadrupole || smallest > 0.0401 * c.cutoff;
   sa.block_half = blocks ? kStrictHalf * c.cutoff : -1.0;
   sa.cut_f = static_cast<float>(c.cutoff);
+  sa.frame = sourceFrame(c);
   sa.accept_half = static_cast<float>(0.04 * c.cutoff * 1.0001);
   sa.sc_r2 = a.wp.inv_4rs2_f * a.poly.scale;
   const bool index = a.tx != nullptr;

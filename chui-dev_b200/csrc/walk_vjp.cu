@@ -53,6 +53,7 @@ struct VjpArgs {
   int targets_per_group;
   int stack_cap, batch_cap;
   float cut_f;
+  SourceFrame frame;
 };
 
 // x_bar_k = G sum_j M(d) (m_k a_bar_j - m_j a_bar_k), d = x_j - x_k, over every
@@ -445,24 +446,28 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, kVjpBlocks) walkVjpGr
         const int j = __ffs(todo) - 1;
         const uint32_t begin = __shfl_sync(0xffffffffu, r.rg.x, j), count = __shfl_sync(0xffffffffu, r.rg.y, j);
         const bool shift = ((moved >> j) & 1u) != 0u, each = ((many >> j) & 1u) != 0u;
-        double jx = 0.0, jy = 0.0, jz = 0.0, ox = 0.0, oy = 0.0, oz = 0.0, rr = 0.0;
+        double jx = 0.0, jy = 0.0, jz = 0.0;
+        int nx = 1, ny = 1, nz = 1;
         if (shift || each) {
           jx = __shfl_sync(0xffffffffu, r.kx, j);
           jy = __shfl_sync(0xffffffffu, r.ky, j);
           jz = __shfl_sync(0xffffffffu, r.kz, j);
         }
         if (each) {
-          ox = __shfl_sync(0xffffffffu, r.ndx, j);
-          oy = __shfl_sync(0xffffffffu, r.ndy, j);
-          oz = __shfl_sync(0xffffffffu, r.ndz, j);
-          rr = static_cast<double>(__shfl_sync(0xffffffffu, rc, j)) * 1.00001;
+          const double h = __shfl_sync(0xffffffffu, r.half, j);
+          nodeImages(w, a.frame, 0, __shfl_sync(0xffffffffu, r.ndx, j), h, f.cx, f.hx, jx, nx);
+          nodeImages(w, a.frame, 1, __shfl_sync(0xffffffffu, r.ndy, j), h, f.cy, f.hy, jy, ny);
+          nodeImages(w, a.frame, 2, __shfl_sync(0xffffffffu, r.ndz, j), h, f.cz, f.hz, jz, nz);
         }
-        for (int im = each ? 0 : 13; im < (each ? 27 : 14); ++im) {
-          const int ix = im / 9 - 1, iy = im / 3 % 3 - 1, iz = im % 3 - 1;
-          if (each && (fabs(ox + ix * w.box[0]) > rr + f.hx || fabs(oy + iy * w.box[1]) > rr + f.hy ||
-                       fabs(oz + iz * w.box[2]) > rr + f.hz))
-            continue;
-          enqueue(begin, count, f.cx + w.box[0] * (jx - ix), f.cy + w.box[1] * (jy - iy), f.cz + w.box[2] * (jz - iz));
+        for (int ix = 0, iy = 0, iz = 0; iz < nz;) {
+          enqueue(begin, count, f.cx + w.box[0] * (jx + ix), f.cy + w.box[1] * (jy + iy), f.cz + w.box[2] * (jz + iz));
+          if (++ix == nx) {
+            ix = 0;
+            if (++iy == ny) {
+              iy = 0;
+              ++iz;
+            }
+          }
         }
       }
     }
@@ -592,6 +597,7 @@ int walkVjpRun(Context& c, int64_t n, const double* sx, const double* sy, const 
   a.batch_cap = kBatchStack;
   a.stack_cap = (kBatchStack + 1 + 7 * std::max<int>(static_cast<int>(c.max_depth), 1) + 7 + 3) & ~3;
   a.cut_f = static_cast<float>(c.cutoff);
+  a.frame = sourceFrame(c);
   const bool eps_zero = !(wp.eps2_f > 1.0e-24f);
   const bool shortp = c.poly.terms <= kPairPolyTerms && c.dpoly.terms <= 12;
 #define CHUI_VJP(EPS, T) return m ? launchVjpGroups<EPS, T, false>(a, s) : launchVjpGroups<EPS, T, true>(a, s)

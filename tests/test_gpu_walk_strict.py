@@ -3,6 +3,8 @@ go wrong: fewer targets than a warp, remainders, meshes so coarse that a pair's
 other image is in reach, targets spread over the box, coincident particles,
 explicit targets, softening lanes, and the sizes around the walk's choice of
 lanes per target -- against the FP64 oracle."""
+import math
+
 import numpy as np
 import pytest
 
@@ -141,3 +143,102 @@ def test_force_vjp_groups(n, mesh, equal):
             out[prec] = torch.stack(s.force_vjp(*p, *cot))
     d = torch.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64]) / torch.linalg.norm(out[ct._abi.FP64])
     assert float(d) <= MIXED
+
+
+def pair_sums(p, box, rs, rcut, eps, rows):
+    """Over the sources j within rcut of each target row: the short-range
+    acceleration sum m K d of the pairs, and the sums m d K_long, m d K_soft and
+    m (r^2 + eps^2)^(-3/2) of the pairs' parts (FP64)."""
+    x, m, L = np.stack(p[:3], 1), p[3], np.array(box)
+    acc, lng, soft, slope = np.zeros((len(rows), 3)), np.zeros(len(rows)), np.zeros(len(rows)), np.zeros(len(rows))
+    for i, row in enumerate(rows):
+        d = x - x[row]
+        d -= L * np.rint(d / L)
+        r2 = (d * d).sum(1)
+        use = (r2 <= rcut * rcut) & (r2 > 0.0)
+        d, r2, mj = d[use], r2[use], m[use]
+        r = np.sqrt(r2)
+        q = r / (2.0 * rs)
+        k_soft = (r2 + eps * eps) ** -1.5
+        k_long = np.where(q < 0.02, 0.752252778 / (8.0 * rs ** 3),
+                          (np.array([math.erf(v) for v in q]) - 2.0 / math.sqrt(math.pi) * q * np.exp(-q * q)) / r ** 3)
+        acc[i] = ((mj * (k_soft - k_long))[:, None] * d).sum(0)
+        lng[i], soft[i], slope[i] = (mj * r * k_long).sum(), (mj * r * k_soft).sum(), (mj * k_soft).sum()
+    return acc, lng, soft, slope
+
+
+def beyond(r, ref, p, box, cell, eps, fp64, rows=None):
+    """The largest error of a target, each against its own allowance: the sums
+    of its own pairs times what each part of a pair is rounded to, and the
+    mesh's rounding. A lost pair of a sparse target is far above it, whatever
+    the accelerations elsewhere in the box.
+      mixed: the long-range polynomial is within 5e-5 of its part of a pair,
+      FP32 products within 1e-6; offsets of up to 3 r_cut are rounded to 24
+      bits, the kernel's slope is at most 2 (r^2 + eps^2)^(-3/2); the FP32 mesh
+      is within 1e-5 of the rms mesh force.
+      FP64: 1e-12 of the parts, offsets to 53 bits of a box length, and the
+      mesh within 1e-11."""
+    rows = np.arange(len(p[0])) if rows is None else rows
+    rs, rcut = 1.25 * cell, 6.25 * cell
+    acc, lng, soft, slope = pair_sums(p, box, rs, rcut, eps, rows)
+    mesh = np.sqrt(((ref.T - acc) ** 2).sum(1).mean())
+    got = np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")])
+    assert np.isfinite(got).all()
+    if fp64:
+        allow = 1e-12 * (lng + soft) + 2.0 * slope * 4.4e-16 * max(box) + 1e-11 * mesh
+    else:
+        allow = 5e-5 * lng + 1e-6 * soft + 2.0 * slope * 2.4e-7 * 3.0 * rcut + 1e-5 * mesh
+    return (np.sqrt(((got - ref) ** 2).sum(0)) / allow).max()
+
+
+# sides in units of 16 mesh cells; r_cut is 0.39 of the shortest
+ELONGATED = [((6, 1, 1), 100, False), ((8, 1, 1), 100, False), ((10, 1, 1), 64, False), ((1, 16, 1), 400, False),
+             ((12, 1, 1), 2000, True), ((6, 1, 6), 1500, True)]
+
+
+def slab(sides, n, blob, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0.0, 1.0, (n, 3)) * np.array(sides)
+    if blob:  # nine tenths in a blob across a corner of the box: the void's leaves are wide
+        k = n - n // 10
+        x[:k] = rng.normal(0.0, 0.08, (k, 3))
+        x = np.mod(x, np.array(sides, dtype=float))
+    return x[:, 0].copy(), x[:, 1].copy(), x[:, 2].copy(), rng.uniform(0.5, 2.0, n)
+
+
+def slab_config(sides, precision, **kw):
+    return ct.TreePmConfig(pm_grid_nx=16 * sides[0], pm_grid_ny=16 * sides[1], pm_grid_nz=16 * sides[2],
+                           box_x=float(sides[0]), box_y=float(sides[1]), box_z=float(sides[2]), opening_theta=0.6,
+                           max_leaf_size=16, softening=0.005, precision=precision, **kw)
+
+
+@pytest.mark.parametrize("sides,n,blob", ELONGATED)
+def test_elongated_boxes(sides, n, blob):
+    """Leaves whose cubes span several short sides of the box: their sources are
+    found at every image, for all targets and for a few."""
+    p = slab(sides, n, blob, n)
+    box, act = [float(v) for v in sides], np.arange(0, n, 7, dtype=np.uint32)
+    for prec, quad in ((ct._abi.MIXED, 1), (ct._abi.FP64, 0)):
+        o = oracle.treepm_solve(*p, oracle.make_params(box=box, mesh=tuple(16 * v for v in sides), theta=0.6, eps=0.005,
+                                                       leaf=16, quadrupole=quad))
+        ref = np.stack([o["ax"], o["ay"], o["az"]])
+        with ct.TreePmCoordinator(slab_config(sides, prec, multipole_order=2 * quad)) as s:
+            fp64 = prec == ct._abi.FP64
+            assert beyond(s.solve_active_set(*p), ref, p, box, 1 / 16, 0.005, fp64) <= 1.0
+            assert beyond(s.solve_active_set(*p, active=act), ref[:, act], p, box, 1 / 16, 0.005, fp64, act) <= 1.0
+
+
+@pytest.mark.parametrize("sides,n,blob", ELONGATED)
+def test_force_vjp_elongated(sides, n, blob):
+    """The mixed adjoint walk in the same boxes against the FP64 adjoint, each
+    particle's gradient on the scale of the median one."""
+    p = [torch.tensor(v, device="cuda") for v in slab(sides, n, blob, n)]
+    g = torch.Generator(device="cpu").manual_seed(n)
+    cot = [torch.randn(n, generator=g, dtype=torch.float64).to("cuda") for _ in range(3)]
+    out = {}
+    for prec in (ct._abi.MIXED, ct._abi.FP64):
+        with ct.TreePmCoordinator(slab_config(sides, prec)) as s:
+            out[prec] = torch.stack(s.force_vjp(*p, *cot))
+    d = torch.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64], dim=0)
+    size = torch.linalg.norm(out[ct._abi.FP64], dim=0)
+    assert float((d / (size + size.median())).max()) <= MIXED
