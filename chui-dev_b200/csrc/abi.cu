@@ -1156,6 +1156,7 @@ static int solveVisitRange(void* handle, const chui_treepm_sources* src, const c
   // queue then carries a lane mask instead of a mass
   wp.uniform_mass = !m || mass_range[0] == mass_range[1];
   wp.m0_f = static_cast<float>(m ? mass_range[0] : src->uniform_mass);
+  wp.m_max = m ? mass_range[1] : src->uniform_mass;
   {
     // group walk eligibility (tree_pm_coupling.cpp:3840-3870, 3922-3925, 4282-4286)
     const double inv_2a2 = (0.25 / c.rs) / c.rs, inv_8a3 = ((0.125 / c.rs) / c.rs) / c.rs;

@@ -62,6 +62,7 @@ struct WalkParams {
   int gauss_lookup;  // Gaussian Hermite table for FP64 direct pairs
   int uniform_mass;  // every source has mass m0
   float m0_f;
+  double m_max;      // the largest source mass
   double angle;    // adaptive_maximum_opening_angle
   double rel_tol;  // relative_force_tolerance
   double floor_;   // relative_force_acceleration_floor_code

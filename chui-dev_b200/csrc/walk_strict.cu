@@ -28,7 +28,7 @@
 // warp straddling a jump of the tree order walked for milliseconds).
 // No lane masks travel with the sources: a target's own entry is at distance
 // zero and adds nothing (targets and sources round the same tree-frame
-// position the same way), sources beyond r_cut fail the pair's cutoff test, and
+// position the same way; EpsForm), sources beyond r_cut fail the pair's cutoff test, and
 // the rare source whose node some target has accepted as a multipole is queued
 // in a batch of its own that those targets' lanes sit out.
 //
@@ -70,6 +70,12 @@ constexpr uint32_t kInBlock = 1u << 31;  // stack entry inside a subtree block (
 constexpr int kBlocks32 = 5;
 
 enum SourceLanes { kUniformMass = 0, kMassLane = 1, kMassEpsLanes = 2 };
+
+// What a target's own entry, and a source that coincides with it, need (FP32,
+// one softening): nothing with kEpsFinite, where the pair's factor m K(0) is a
+// finite number times d = 0; otherwise the pair loop drops pairs at distance
+// zero, on r^2 itself (kEpsGuard: two more instructions per two pairs).
+enum EpsForm { kEpsNone = 0, kEpsFinite = 1, kEpsGuard = 2 };
 
 // A target's position: its source's tree-frame position, or the explicit one.
 __device__ __forceinline__ void targetPosition(const WalkArgs& a, int64_t v, uint32_t slot, uint32_t row, double& x,
@@ -186,10 +192,13 @@ struct WarpShared {
 
 // kTerms: terms of the long-range coefficient's polynomial; FP64 with 0: the
 // reference's erf/exp form (or its Gaussian table).
-template <class Real, bool kEpsZero, int kTerms, int kLanes, bool kIndex>
+template <class Real, int kEps, int kTerms, int kLanes, bool kIndex>
 __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? kBlocks32 : 4)
     walkStrictKernel(WalkArgs a, StrictArgs sa) {
   constexpr bool kF64 = sizeof(Real) == 8;
+  constexpr bool kEpsZero = kEps == kEpsNone;
+  constexpr bool kPairEps = kLanes == kMassEpsLanes;      // FP32: softening per pair
+  constexpr bool kFolded = !kPairEps && kEps == kEpsFinite;  // FP32: r^2 + eps^2 in one chain
   using Shared = WarpShared<Real, kLanes, kIndex>;
   constexpr int kQ = Shared::kQ;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -316,30 +325,33 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
           const float2 dy = __fadd2_rn(sy, nty);
           const float2 dz = __fadd2_rn(sz, ntz);
           // r^2 + eps^2 in one chain (eps^2 folded into the cutoff test and the
-          // polynomial variable); per-pair softening keeps r^2 apart
+          // polynomial variable), or r^2 apart
           float2 r2e, r2;
-          if constexpr (kLanes == kMassEpsLanes) {
-            r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-            const float2 ep = make_float2(fmaxf(es.x, eps_f), fmaxf(es.y, eps_f));
-            r2e = __ffma2_rn(ep, ep, r2);
-          } else {
-            r2e = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, kEpsZero ? __fmul2_rn(dz, dz) : __ffma2_rn(dz, dz, a.eps2_2)));
+          if constexpr (kFolded) {
+            r2e = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, a.eps2_2)));
             r2 = r2e;
+          } else {
+            r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+            r2e = r2;
+            if constexpr (kPairEps) {
+              const float2 ep = make_float2(fmaxf(es.x, eps_f), fmaxf(es.y, eps_f));
+              r2e = __ffma2_rn(ep, ep, r2);
+            } else if constexpr (kEps == kEpsGuard) {
+              r2e = __fadd2_rn(r2, a.eps2_2);
+            }
           }
-          const float cut_t = kLanes == kMassEpsLanes || kEpsZero ? cut2 : a.cut2e;
+          const float cut_t = kFolded ? a.cut2e : cut2;
           bool in0 = r2.x <= cut_t, in1 = r2.y <= cut_t;
           if constexpr (kIndex) {
             in0 = in0 && ok0;
             in1 = in1 && ok1;
           }
-          // coincident particles add nothing: d = 0 with a finite kernel, or
-          // excluded where the kernel is infinite there
-          if constexpr (kEpsZero || kLanes == kMassEpsLanes) {
+          // coincident particles add nothing
+          if constexpr (!kFolded) {
             in0 = in0 && r2.x > 0.f;
             in1 = in1 && r2.y > 0.f;
           }
-          const float2 klong = hornerR2x2<kTerms>(a.pk2, r2, a.sc2,
-                                                  kLanes == kMassEpsLanes || kEpsZero ? a.mone2 : a.soff2);
+          const float2 klong = hornerR2x2<kTerms>(a.pk2, r2, a.sc2, kFolded ? a.soff2 : a.mone2);
           const float2 rinv = make_float2(rsqrtf(r2e.x), rsqrtf(r2e.y));
           float2 k3 = __ffma2_rn(__fmul2_rn(rinv, rinv), rinv, klong);  // K_soft - K_long
           if constexpr (kLanes >= kMassLane) k3 = __fmul2_rn(k3, m);
@@ -691,9 +703,9 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
   }
 }
 
-template <class Real, bool kEpsZero, int kTerms, int kLanes, bool kIndex>
+template <class Real, int kEps, int kTerms, int kLanes, bool kIndex>
 int launchStrict(const WalkArgs& a, const StrictArgs& sa, cudaStream_t s) {
-  auto kernel = walkStrictKernel<Real, kEpsZero, kTerms, kLanes, kIndex>;
+  auto kernel = walkStrictKernel<Real, kEps, kTerms, kLanes, kIndex>;
   const size_t smem = kWalkWarpsPerBlock * WarpShared<Real, kLanes, kIndex>::bytes(sa.stack_cap);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return CHUI_TREEPM_EDEVICE;
@@ -768,29 +780,34 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
     sa.h64_scale = p.scale * 0.25 / (c.rs * c.rs);
     const int terms = a.wp.gauss_lookup || !std::isfinite(k) ? 0 : p.terms;
     sa.caller_sources = tiny ? 1 : 0;
-#define CHUI_STRICT64(T) return launchStrict<double, false, T, kMassEpsLanes, true>(a, sa, s)
+#define CHUI_STRICT64(T) return launchStrict<double, kEpsGuard, T, kMassEpsLanes, true>(a, sa, s)
     if (terms > kPoly64Short) CHUI_STRICT64(kPoly64Max);
     if (terms > 0) CHUI_STRICT64(kPoly64Short);
     CHUI_STRICT64(0);
 #undef CHUI_STRICT64
   }
   if (soft)
-    return index ? launchStrict<float, false, kPolyMaxTerms, kMassEpsLanes, true>(a, sa, s)
-                 : launchStrict<float, false, kPolyMaxTerms, kMassEpsLanes, false>(a, sa, s);
+    return index ? launchStrict<float, kEpsGuard, kPolyMaxTerms, kMassEpsLanes, true>(a, sa, s)
+                 : launchStrict<float, kEpsGuard, kPolyMaxTerms, kMassEpsLanes, false>(a, sa, s);
   // a softening whose FP32 kernel would overflow at distance zero counts as none
   const float e2 = a.wp.eps2_f;
   const bool eps_zero = !(e2 > 1.0e-24f);
   const bool shortp = a.poly.terms <= kPairPolyTerms;
+  // m K(0) = m (eps^-3 - 0.094 / r_s^3) of the heaviest source must be well
+  // inside FP32 (a source's mass is a factor of each pair, a common mass is not)
+  const double heaviest = std::max(1.0, a.wp.m_max);
+  const bool finite = heaviest * (std::pow(a.wp.eps, -3.0) + 0.1 / (c.rs * c.rs * c.rs)) < 1.0e36;
 #define CHUI_STRICT32(EPS, T)                                                                       \
   return index ? launchStrict<float, EPS, T, kMassLane, true>(a, sa, s)                             \
                : (a.wp.uniform_mass ? launchStrict<float, EPS, T, kUniformMass, false>(a, sa, s)    \
                                     : launchStrict<float, EPS, T, kMassLane, false>(a, sa, s))
   if (eps_zero) {
-    if (shortp) CHUI_STRICT32(true, kPairPolyTerms);
-    CHUI_STRICT32(true, kPolyMaxTerms);
+    if (shortp) CHUI_STRICT32(kEpsNone, kPairPolyTerms);
+    CHUI_STRICT32(kEpsNone, kPolyMaxTerms);
   }
-  if (shortp) CHUI_STRICT32(false, kPairPolyTerms);
-  CHUI_STRICT32(false, kPolyMaxTerms);
+  if (!finite) CHUI_STRICT32(kEpsGuard, kPolyMaxTerms);
+  if (shortp) CHUI_STRICT32(kEpsFinite, kPairPolyTerms);
+  CHUI_STRICT32(kEpsFinite, kPolyMaxTerms);
 #undef CHUI_STRICT32
 }
 

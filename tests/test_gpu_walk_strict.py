@@ -43,7 +43,7 @@ def particles(n, seed):
 
 def config(mesh, precision, **kw):
     return ct.TreePmConfig(pm_grid_nx=mesh, pm_grid_ny=mesh, pm_grid_nz=mesh, box_x=BOX[0], box_y=BOX[1], box_z=BOX[2],
-                           opening_theta=0.6, max_leaf_size=16, softening=0.05, precision=precision, **kw)
+                           opening_theta=0.6, max_leaf_size=16, precision=precision, **dict(dict(softening=0.05), **kw))
 
 
 def reference(p, mesh, active=None, quadrupole=1):
@@ -242,3 +242,25 @@ def test_force_vjp_elongated(sides, n, blob):
     d = torch.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64], dim=0)
     size = torch.linalg.norm(out[ct._abi.FP64], dim=0)
     assert float((d / (size + size.median())).max()) <= MIXED
+
+
+@pytest.mark.parametrize("equal", [False, True])
+@pytest.mark.parametrize("eps", [1e-10, 1e-13])
+def test_tiny_softening_and_heavy_masses(eps, equal):
+    """m / eps^3 beyond FP32 with a softening that is only a guard: a target's
+    own entry and a coincident particle still add nothing (full, active and
+    explicit targets)."""
+    n = 4000
+    p = list(particles(n, 11))
+    p[3] = np.full(n, 3.0e9) if equal else 10.0 ** np.random.default_rng(1).uniform(0.0, 10.0, n)
+    act = np.arange(3, n, 11, dtype=np.uint32)
+    t = (p[0][act] + BOX[0], p[1][act], p[2][act])
+    cfg = dict(softening=eps)
+    cell = (BOX[0] * BOX[1] * BOX[2]) ** (1 / 3) / 48
+    with ct.TreePmCoordinator(config(48, ct._abi.FP64, **cfg)) as s:
+        r = s.solve_active_set(*p)
+    ref = np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")])
+    with ct.TreePmCoordinator(config(48, ct._abi.MIXED, **cfg)) as s:
+        assert beyond(s.solve_active_set(*p), ref, p, BOX, cell, eps, False) <= 1.0
+        assert beyond(s.solve_active_set(*p, active=act), ref[:, act], p, BOX, cell, eps, False, act) <= 1.0
+        assert beyond(s.solve_active_set(*p, active=act, targets=t), ref[:, act], p, BOX, cell, eps, False, act) <= 1.0
