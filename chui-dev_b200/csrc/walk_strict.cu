@@ -789,9 +789,7 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
   if (soft)
     return index ? launchStrict<float, kEpsGuard, kPolyMaxTerms, kMassEpsLanes, true>(a, sa, s)
                  : launchStrict<float, kEpsGuard, kPolyMaxTerms, kMassEpsLanes, false>(a, sa, s);
-  // a softening whose FP32 kernel would overflow at distance zero counts as none
-  const float e2 = a.wp.eps2_f;
-  const bool eps_zero = !(e2 > 1.0e-24f);
+  const bool eps_zero = a.wp.eps == 0.0;
   const bool shortp = a.poly.terms <= kPairPolyTerms;
   // m K(0) = m (eps^-3 - 0.094 / r_s^3) of the heaviest source must be well
   // inside FP32 (a source's mass is a factor of each pair, a common mass is not)

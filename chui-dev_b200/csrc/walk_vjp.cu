@@ -598,7 +598,7 @@ int walkVjpRun(Context& c, int64_t n, const double* sx, const double* sy, const 
   a.stack_cap = (kBatchStack + 1 + 7 * std::max<int>(static_cast<int>(c.max_depth), 1) + 7 + 3) & ~3;
   a.cut_f = static_cast<float>(c.cutoff);
   a.frame = sourceFrame(c);
-  const bool eps_zero = !(wp.eps2_f > 1.0e-24f);
+  const bool eps_zero = wp.eps == 0.0;
   const bool shortp = c.poly.terms <= kPairPolyTerms && c.dpoly.terms <= 12;
 #define CHUI_VJP(EPS, T) return m ? launchVjpGroups<EPS, T, false>(a, s) : launchVjpGroups<EPS, T, true>(a, s)
   if (eps_zero) {

@@ -42,8 +42,9 @@ def particles(n, seed):
 
 
 def config(mesh, precision, **kw):
-    return ct.TreePmConfig(pm_grid_nx=mesh, pm_grid_ny=mesh, pm_grid_nz=mesh, box_x=BOX[0], box_y=BOX[1], box_z=BOX[2],
-                           opening_theta=0.6, max_leaf_size=16, precision=precision, **dict(dict(softening=0.05), **kw))
+    return ct.TreePmConfig(pm_grid_nx=mesh, pm_grid_ny=mesh, pm_grid_nz=mesh, opening_theta=0.6, max_leaf_size=16,
+                           precision=precision,
+                           **dict(dict(box_x=BOX[0], box_y=BOX[1], box_z=BOX[2], softening=0.05), **kw))
 
 
 def reference(p, mesh, active=None, quadrupole=1):
@@ -264,3 +265,23 @@ def test_tiny_softening_and_heavy_masses(eps, equal):
         assert beyond(s.solve_active_set(*p), ref, p, BOX, cell, eps, False) <= 1.0
         assert beyond(s.solve_active_set(*p, active=act), ref[:, act], p, BOX, cell, eps, False, act) <= 1.0
         assert beyond(s.solve_active_set(*p, active=act, targets=t), ref[:, act], p, BOX, cell, eps, False, act) <= 1.0
+
+
+def test_softening_in_small_units():
+    """A softening below 1e-12 in a box of 1e-9 is a softening like any other:
+    a blob of its size against the FP64 walk."""
+    n, unit, eps = 4000, 1e-10, 9e-13
+    p = list(particles(n, 5))
+    rng = np.random.default_rng(2)
+    for k in range(3):
+        p[k][:500] = 0.6 * BOX[k] + rng.normal(0.0, 0.02, 500)
+        p[k] *= unit
+    cfg = dict(softening=eps, box_x=BOX[0] * unit, box_y=BOX[1] * unit, box_z=BOX[2] * unit)
+    out = {}
+    for prec in (ct._abi.MIXED, ct._abi.FP64):
+        with ct.TreePmCoordinator(config(48, prec, **cfg)) as s:
+            r = s.solve_active_set(*p)
+            out[prec] = np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")])
+    size = np.linalg.norm(out[ct._abi.FP64], axis=0)
+    d = np.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64], axis=0)
+    assert (d / (size + np.median(size))).max() <= MIXED
