@@ -100,7 +100,8 @@ struct StrictArgs {
   float sc_r2;                  // r^2 -> polynomial variable
   double h64[kPoly64Max];       // FP64: H(t)/(8 r_s^3) in s = r^2 h64_scale - 1
   double h64_scale;
-  int caller_sources;           // FP64: sources at the caller's coordinates instead of the tree frame's
+  int canonical;                // FP64: every coordinate lies in [0, L)
+  double anchor[3];             // ... and the tree frame moves those below the anchor up by L
   SourceFrame frame;
 };
 

@@ -99,10 +99,23 @@ __device__ __forceinline__ double targetOffset(const WalkArgs& a, double d, int 
   return a.tx ? frameImage(d, a.wp.box[axis], a.wp.inv_box[axis]) : d;
 }
 
-// Offset of a source at the caller's coordinate, moved by whole box lengths to
-// the image at (about) `near`.
-__device__ __forceinline__ double callerOffset(double d, double near, double length, double inv_length) {
-  return length > 0.0 ? fma(length, rint((near - d) * inv_length), d) : d;
+// FP64: c + q L in two parts {hi, lo}, so that p - c - q L of a position p at the
+// caller's coordinate is (p - hi) - lo, rounded on the scale of the offset (p lies
+// near hi). The tree frame's copy of a position below the anchor is p + L rounded
+// to an ulp of L, which is no rounding for a close pair; formed this way for
+// targets and sources alike, coincident particles are at distance zero.
+__device__ __forceinline__ double2 movedOrigin(double c, double q, double length) {
+  const double ql = __dmul_rn(q, length);
+  const double hi = __dadd_rn(c, ql);
+  const double part = __dsub_rn(hi, c);
+  return make_double2(hi, __dadd_rn(__dsub_rn(c, __dsub_rn(hi, part)), __dsub_rn(ql, part)));
+}
+
+// FP64: offset from c of a position at the caller's coordinate p, at the image at
+// (about) `near`.
+__device__ __forceinline__ double callerOffset(double p, double near, double c, double length, double inv_length) {
+  const double2 o = movedOrigin(c, length > 0.0 ? rint(((p - c) - near) * inv_length) : 0.0, length);
+  return __dsub_rn(__dsub_rn(p, o.x), o.y);
 }
 
 // Cuts each run of 32 visit positions into groups: maximal runs of consecutive
@@ -187,7 +200,11 @@ struct WarpShared {
   static constexpr size_t kArrays = 3 + (kLanes >= kMassLane ? 1 : 0) + (kLanes >= kMassEpsLanes ? 1 : 0);
   __host__ __device__ static constexpr size_t queueBytes() { return kArrays * kQ * sizeof(Real) + (kIndex ? kQ * sizeof(uint32_t) : 0); }
   __host__ __device__ static constexpr size_t accBytes() { return 3 * 32 * sizeof(double); }
-  __host__ __device__ static constexpr size_t bytes(int stack_cap) { return queueBytes() + accBytes() + static_cast<size_t>(stack_cap) * 8; }
+  // FP64: the sources' origin per axis, for positions the tree frame keeps and moves
+  __host__ __device__ static constexpr size_t originBytes() { return sizeof(Real) == 8 ? 6 * sizeof(double2) : 0; }
+  __host__ __device__ static constexpr size_t bytes(int stack_cap) {
+    return queueBytes() + accBytes() + originBytes() + static_cast<size_t>(stack_cap) * 8;
+  }
 };
 
 // kTerms: terms of the long-range coefficient's polynomial; FP64 with 0: the
@@ -211,7 +228,8 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
   Real* qe = qm + kQ;  // kLanes >= kMassEpsLanes
   uint32_t* qi = reinterpret_cast<uint32_t*>(mine + Shared::kArrays * kQ * sizeof(Real));
   double* acc = reinterpret_cast<double*>(mine + Shared::queueBytes());
-  uint32_t* stack = reinterpret_cast<uint32_t*>(mine + Shared::queueBytes() + Shared::accBytes());
+  double2* origin = reinterpret_cast<double2*>(mine + Shared::queueBytes() + Shared::accBytes());  // FP64
+  uint32_t* stack = reinterpret_cast<uint32_t*>(mine + Shared::queueBytes() + Shared::accBytes() + Shared::originBytes());
   uint32_t* stack_mask = stack + sa.stack_cap;
 
   const WalkParams& w = a.wp;
@@ -243,8 +261,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       row = a.active ? a.active[slot] : slot;
       targetPosition(a, v, slot, row, px, py, pz);
     }
-    // FP64 takes targets at the caller's coordinates (the tree frame rounds a
-    // position that it moves by a box length)
+    // FP64 takes targets and sources at the caller's coordinates (callerOffset)
     const double ux = px, uy = py, uz = pz;
     if constexpr (kF64) {
       if (valid && !a.tx) {
@@ -280,12 +297,18 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
     }
     const float bx = static_cast<float>(cx - fx0), by = static_cast<float>(cy - fy0), bz = static_cast<float>(cz - fz0);
     // target offsets from the origin: the arithmetic of the queued sources, so
-    // in FP32 a target meets its own entry at distance exactly zero
+    // a target meets its own entry at distance exactly zero
     Real tx = Real(0), ty = Real(0), tz = Real(0);
     if (valid) {
-      tx = static_cast<Real>(kF64 ? frameImage(px - fx0, w.box[0], w.inv_box[0]) : targetOffset(a, px - fx0, 0));
-      ty = static_cast<Real>(kF64 ? frameImage(py - fy0, w.box[1], w.inv_box[1]) : targetOffset(a, py - fy0, 1));
-      tz = static_cast<Real>(kF64 ? frameImage(pz - fz0, w.box[2], w.inv_box[2]) : targetOffset(a, pz - fz0, 2));
+      if constexpr (kF64) {
+        tx = callerOffset(px, targetOffset(a, ux - cx, 0), cx, w.box[0], w.inv_box[0]);
+        ty = callerOffset(py, targetOffset(a, uy - cy, 1), cy, w.box[1], w.inv_box[1]);
+        tz = callerOffset(pz, targetOffset(a, uz - cz, 2), cz, w.box[2], w.inv_box[2]);
+      } else {
+        tx = static_cast<Real>(targetOffset(a, px - fx0, 0));
+        ty = static_cast<Real>(targetOffset(a, py - fy0, 1));
+        tz = static_cast<Real>(targetOffset(a, pz - fz0, 2));
+      }
     }
     const double eps_d = kLanes == kMassEpsLanes ? targetEps(a, slot, row, valid) : w.eps;
     const float eps_f = static_cast<float>(eps_d);
@@ -418,11 +441,26 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       __syncwarp();
     };
 
+    // FP64: the sources' origin at the image (ix, iy, iz)
+    auto setOrigin = [&](double ix, double iy, double iz) {
+      if (lane < 6) {
+        const int axis = lane >> 1;
+        origin[lane] = movedOrigin(axis == 0 ? cx : (axis == 1 ? cy : cz),
+                                   (axis == 0 ? ix : (axis == 1 ? iy : iz)) - (lane & 1),
+                                   axis == 0 ? w.box[0] : (axis == 1 ? w.box[1] : w.box[2]));
+      }
+      __syncwarp();
+    };
+
     // Queue the sources [begin, begin + count) within r_cut of the box, as
-    // offsets from (sx, sy, sz): the box centre moved to the sources' image.
-    // `lanes` take them; `inside`: every one is within r_cut of every target.
-    auto enqueue = [&](uint32_t begin, uint32_t count, uint32_t lanes, bool inside, double sx, double sy, double sz) {
-      const double4* src = a.src_u4 + begin;
+    // offsets from the origin moved by (ix, iy, iz) box lengths to the sources'
+    // image. `lanes` take them; `inside`: every one is within r_cut of every target.
+    auto enqueue = [&](uint32_t begin, uint32_t count, uint32_t lanes, bool inside, double ix, double iy, double iz) {
+      const bool caller = kF64 && sa.canonical != 0;  // positions as the caller gave them
+      const double4* src = (caller ? a.src_d4 : a.src_u4) + begin;
+      // unmoved sources keep the origin's bits (FP32: a target's own entry stays at
+      // distance zero)
+      const double sx = fx0 + w.box[0] * ix, sy = fy0 + w.box[1] * iy, sz = fz0 + w.box[2] * iz;
       // rounding of the box's position in the frame
       const float slack = 2.4e-7f * fmaxf(fabsf(bx), fmaxf(fabsf(by), fabsf(bz)));
       uint32_t k = lane;
@@ -438,12 +476,19 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
         on = lanes;
         double dx = cur.x - sx, dy = cur.y - sy, dz = cur.z - sz;
         if constexpr (kF64) {
-          if (sa.caller_sources && have) {
-            // the caller's coordinates at the same image
+          if (caller) {
+            // a position below the anchor is a box length further up in the tree frame
+            const double2 px0 = origin[cur.x < sa.anchor[0] ? 1 : 0], py0 = origin[cur.y < sa.anchor[1] ? 3 : 2],
+                          pz0 = origin[cur.z < sa.anchor[2] ? 5 : 4];
+            dx = __dsub_rn(__dsub_rn(cur.x, px0.x), px0.y);
+            dy = __dsub_rn(__dsub_rn(cur.y, py0.x), py0.y);
+            dz = __dsub_rn(__dsub_rn(cur.z, pz0.x), pz0.y);
+          } else if (have) {
+            // coordinates outside the box: the image the tree frame took
             const double4 p = a.src_d4[pos];
-            dx = callerOffset(p.x - cx, dx, w.box[0], w.inv_box[0]);
-            dy = callerOffset(p.y - cy, dy, w.box[1], w.inv_box[1]);
-            dz = callerOffset(p.z - cz, dz, w.box[2], w.inv_box[2]);
+            dx = callerOffset(p.x, dx, cx, w.box[0], w.inv_box[0]);
+            dy = callerOffset(p.y, dy, cy, w.box[1], w.inv_box[1]);
+            dz = callerOffset(p.z, dz, cz, w.box[2], w.inv_box[2]);
           }
         }
         const float ex = static_cast<float>(dx), ey = static_cast<float>(dy), ez = static_cast<float>(dz);
@@ -474,6 +519,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
       }
     };
 
+    if constexpr (kF64) setOrigin(0.0, 0.0, 0.0);
     bool overflow = false;
     while (sp > 0) {
       // take up to 32 nodes, leaving room for a depth-first descent below them
@@ -669,10 +715,10 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
           nodeImages(w, sa.frame, 2, __shfl_sync(0xffffffffu, r.ndz, j), h, cz, hbz, jz, nz);
         }
         for (int ix = 0, iy = 0, iz = 0; iz < nz;) {
-          // unmoved sources keep the origin's bits (a target's own entry stays at
-          // distance zero)
-          enqueue(begin, count, lanes, !each && ((within >> j) & 1u) != 0u, fx0 + w.box[0] * (jx + ix),
-                  fy0 + w.box[1] * (jy + iy), fz0 + w.box[2] * (jz + iz));
+          if constexpr (kF64) {
+            if (shift || each) setOrigin(jx + ix, jy + iy, jz + iz);
+          }
+          enqueue(begin, count, lanes, !each && ((within >> j) & 1u) != 0u, jx + ix, jy + iy, jz + iz);
           if (++ix == nx) {
             ix = 0;
             if (++iy == ny) {
@@ -680,6 +726,9 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
               ++iz;
             }
           }
+        }
+        if constexpr (kF64) {
+          if (shift || each) setOrigin(0.0, 0.0, 0.0);
         }
       }
     }
@@ -778,8 +827,13 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
     const double k = 0.125 / (c.rs * c.rs * c.rs);
     for (int j = 0; j < kPoly64Max; ++j) sa.h64[j] = p.c[j] * k;
     sa.h64_scale = p.scale * 0.25 / (c.rs * c.rs);
+    sa.canonical = 1;
+    for (int a0 = 0; a0 < 3; ++a0) {
+      const double L = a.wp.box[a0];
+      if (L > 0.0 && !(a.wp.src_lo[a0] >= 0.0 && a.wp.src_hi[a0] < L)) sa.canonical = 0;
+      sa.anchor[a0] = L > 0.0 ? c.tree_anchor[a0] : -INFINITY;
+    }
     const int terms = a.wp.gauss_lookup || !std::isfinite(k) ? 0 : p.terms;
-    sa.caller_sources = tiny ? 1 : 0;
 #define CHUI_STRICT64(T) return launchStrict<double, kEpsGuard, T, kMassEpsLanes, true>(a, sa, s)
     if (terms > kPoly64Short) CHUI_STRICT64(kPoly64Max);
     if (terms > 0) CHUI_STRICT64(kPoly64Short);

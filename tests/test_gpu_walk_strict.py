@@ -285,3 +285,35 @@ def test_softening_in_small_units():
     size = np.linalg.norm(out[ct._abi.FP64], axis=0)
     d = np.linalg.norm(out[ct._abi.MIXED] - out[ct._abi.FP64], axis=0)
     assert (d / (size + np.median(size))).max() <= MIXED
+
+
+@pytest.mark.parametrize("away", [0, 1])
+def test_fp64_coincident_and_close_pairs(away):
+    """FP64 without softening: particles that coincide add nothing to each other,
+    and pairs a few hundred ulps of the box length apart keep their separation,
+    on either side of the tree frame's seam (the positions it moves by a box
+    length are rounded there); away: every coordinate outside the box."""
+    n = 4000
+    p = list(particles(n, 17))
+    rng = np.random.default_rng(4)
+    at = rng.permutation(n)[:1200]
+    for k in range(3):
+        p[k][at[600:]] = p[k][at[:600]]  # 600 pairs, coincident
+    far = at[900:]  # the last 300 of them 0.02 .. 0.5 * 2^-40 apart on each axis
+    for k in range(3):
+        p[k][far] = np.mod(p[k][far] + rng.uniform(0.02, 0.5, 300) * 2.0 ** -40, BOX[k])
+        p[k] += away * (1, -2, 3)[k] * BOX[k]
+    o = oracle.treepm_solve(*p, oracle.make_params(box=BOX, mesh=(48,) * 3, theta=0.6, eps=0.0, leaf=16, quadrupole=0))
+    ref = np.stack([o["ax"], o["ay"], o["az"]])
+    with ct.TreePmCoordinator(config(48, ct._abi.FP64, multipole_order=0, softening=0.0)) as s:
+        for rows in (np.arange(n), at.astype(np.uint32)):
+            r = s.solve_active_set(*p) if len(rows) == n else s.solve_active_set(*p, active=rows)
+            got = np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")])
+            assert np.isfinite(got).all()
+            size = np.linalg.norm(ref[:, rows], axis=0)
+            # a close pair's separation is exact up to 2^-53 of the offsets it is the
+            # difference of (below 4 box-lengths / 10): 1e-3 of 2^-45 and more
+            assert (np.linalg.norm(got - ref[:, rows], axis=0) <= 1e-3 * size + 1e-11 * np.median(size)).all()
+            alone = ~np.isin(rows, at[300:600]) & ~np.isin(rows, far)
+            scale = size[alone] + np.median(size)
+            assert (np.linalg.norm(got - ref[:, rows], axis=0)[alone] / scale).max() <= 1e-11
