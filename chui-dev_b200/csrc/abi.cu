@@ -439,54 +439,6 @@ PolyH fitChebyshev(F func, double t_cut, double tolerance = 2.0e-6, int short_te
 #endif
 PolyH fitPoly(double t_cut) { return fitChebyshev(hostH, t_cut, CHUI_PAIR_TOLERANCE, kPairPolyTerms); }
 
-// H in FP64 for the FP64 pair loops: Chebyshev interpolation on [0, t_cut]
-// (long double on the host), accepted when it is within 4e-16 of H everywhere
-// (H(0) = 0.75): the closed form's erf - exp difference loses 1e-13 of it at
-// small t. 20 terms reach that for r_cut / r_s up to 5, 32 up to 10.
-PolyH64 fitPoly64(double t_cut) {
-  const long double pi = 3.141592653589793238462643383279502884L;
-  // H(t) = (4/sqrt(pi)) e^-t sum_k (2t)^k / (3 5 ... (2k+3)): positive terms
-  auto exactH = [&](long double t) {
-    long double sum = 0.0L, term = 1.0L / 3.0L;
-    for (int k = 1; k < 400 && term > 1e-22L * sum; ++k) {
-      sum += term;
-      term *= 2.0L * t / (2.0L * k + 3.0L);
-    }
-    return 4.0L / std::sqrt(pi) * std::exp(-t) * sum;
-  };
-  for (const int m : {kPoly64Short, kPoly64Max}) {
-    std::vector<long double> f(m), mono(m, 0.0L), tkm1(m, 0.0L), tk(m, 0.0L), tkp1(m, 0.0L);
-    for (int k = 0; k < m; ++k) f[k] = exactH((std::cos(pi * (k + 0.5L) / m) + 1.0L) * 0.5L * t_cut);
-    tkm1[0] = 1.0L;
-    tk[1] = 1.0L;
-    for (int j = 0; j < m; ++j) {
-      long double sum = 0.0L;
-      for (int k = 0; k < m; ++k) sum += f[k] * std::cos(pi * j * (k + 0.5L) / m);
-      const long double cheb = (j == 0 ? 1.0L : 2.0L) * sum / m;
-      if (j >= 2) {
-        for (int i = m - 1; i >= 0; --i) tkp1[i] = (i > 0 ? 2.0L * tk[i - 1] : 0.0L) - tkm1[i];
-        tkm1 = tk;
-        tk = tkp1;
-      }
-      const std::vector<long double>& poly = j == 0 ? tkm1 : tk;
-      for (int i = 0; i < m; ++i) mono[i] += cheb * poly[i];
-    }
-    PolyH64 p;
-    p.terms = m;
-    p.scale = 2.0 / t_cut;
-    for (int i = 0; i < m; ++i) p.c[i] = static_cast<double>(mono[i]);
-    double err = 0.0;
-    for (int k = 0; k <= 96; ++k) {  // several points to each of the fit's oscillations
-      const double t = t_cut * k / 96.0, s = std::fma(t, p.scale, -1.0);
-      double h = p.c[m - 1];
-      for (int i = m - 2; i >= 0; --i) h = std::fma(h, s, p.c[i]);
-      err = std::max(err, std::fabs(static_cast<double>(static_cast<long double>(h) - exactH(t))));
-    }
-    if (err <= 4.0e-16) return p;
-  }
-  return PolyH64();
-}
-
 int fail(Context& c, int code, const std::string& msg) {
   c.last_error = msg;
   return code;
@@ -590,7 +542,7 @@ void applyConfig(Context& c, const chui_treepm_config& cfg) {
   c.cutoff = cfg.rcut_cells * c.spacing;
   const double t_cut = (c.cutoff * c.cutoff) / (4.0 * c.rs * c.rs) * (1.0 + 1.0e-5);
   c.poly = fitPoly(t_cut);
-  c.poly64 = fitPoly64(t_cut);
+  c.poly64 = fitPoly64(c.rs, c.cutoff);
   c.dpoly = fitChebyshev(hostHp, t_cut);
   // H'' scales the quadrupole's second-derivative term only: 1e-5 suffices
   c.ddpoly = fitChebyshev(hostHpp, t_cut, 1.0e-5);

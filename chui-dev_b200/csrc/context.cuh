@@ -11,6 +11,7 @@
 
 #include "../../include/chui_treepm.h"
 #include "common.cuh"
+#include "pair64.hpp"
 
 namespace chui {
 
@@ -32,15 +33,6 @@ struct PolyH {
   float scale = 0.f;          // 2 / t_cut
   float c[kPolyMaxTerms] = {};
   double max_rel_error = 0.0;
-};
-
-// FP64 coefficients of H(t) in s = t*scale - 1 on [0, t_cut]; terms 0: no fit
-// reaches FP64 accuracy (very large r_cut / r_s).
-constexpr int kPoly64Short = 20, kPoly64Max = 32;
-struct PolyH64 {
-  int terms = 0;
-  double scale = 0.0;
-  double c[kPoly64Max] = {};
 };
 
 // Per-solve scalar geometry shared with the walk kernel.

@@ -98,7 +98,7 @@ struct StrictArgs {
   float cut_f;                  // r_cut
   float accept_half;            // nodes from this half-size on are never accepted as multipoles
   float sc_r2;                  // r^2 -> polynomial variable
-  double h64[kPoly64Max];       // FP64: H(t)/(8 r_s^3) in s = r^2 h64_scale - 1
+  double h64[kPoly64Terms];     // FP64: H(t)/(8 r_s^3) in s = 1 - r^2 h64_scale
   double h64_scale;
   int canonical;                // FP64: every coordinate lies in [0, L)
   double anchor[3];             // ... and the tree frame moves those below the anchor up by L

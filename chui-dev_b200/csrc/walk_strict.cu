@@ -415,14 +415,7 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32, sizeof(Real) == 4 ? k
           const double pe = fmax(qe[k], eps_d);
           double kr;
           if constexpr (kTerms > 0) {
-            const double s = fma(r2, sa.h64_scale, -1.0);
-            double h = sa.h64[kTerms - 1];
-#pragma unroll
-            for (int j = kTerms - 2; j >= 0; --j) h = fma(h, s, sa.h64[j]);
-            const double d = fma(pe, pe, r2);
-            double ri = rsqrt(d);
-            ri = fma(0.5 * ri, fma(-d * ri, ri, 1.0), ri);  // to half an ulp: it is cubed
-            kr = fma(ri * ri, ri, -h);                      // h64 carries the 1/(8 r_s^3)
+            kr = softMinusLong64(r2, pe, sa.h64_scale, sa.h64);
           } else {
             kr = !in ? 0.0 : (w.gauss_lookup ? gaussResidualInvR3(a, r2, pe) : residualInvR3(r2, pe, w.rs));
           }
@@ -823,22 +816,17 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
   const bool index = a.tx != nullptr;
   const bool soft = a.src_eps || a.tgt_eps;
   if (f64) {
-    const PolyH64& p = c.poly64;
-    const double k = 0.125 / (c.rs * c.rs * c.rs);
-    for (int j = 0; j < kPoly64Max; ++j) sa.h64[j] = p.c[j] * k;
-    sa.h64_scale = p.scale * 0.25 / (c.rs * c.rs);
+    for (int j = 0; j < kPoly64Terms; ++j) sa.h64[j] = c.poly64.c[j];
+    sa.h64_scale = c.poly64.scale;
     sa.canonical = 1;
     for (int a0 = 0; a0 < 3; ++a0) {
       const double L = a.wp.box[a0];
       if (L > 0.0 && !(a.wp.src_lo[a0] >= 0.0 && a.wp.src_hi[a0] < L)) sa.canonical = 0;
       sa.anchor[a0] = L > 0.0 ? c.tree_anchor[a0] : -INFINITY;
     }
-    const int terms = a.wp.gauss_lookup || !std::isfinite(k) ? 0 : p.terms;
-#define CHUI_STRICT64(T) return launchStrict<double, kEpsGuard, T, kMassEpsLanes, true>(a, sa, s)
-    if (terms > kPoly64Short) CHUI_STRICT64(kPoly64Max);
-    if (terms > 0) CHUI_STRICT64(kPoly64Short);
-    CHUI_STRICT64(0);
-#undef CHUI_STRICT64
+    return a.wp.gauss_lookup || c.poly64.terms == 0
+               ? launchStrict<double, kEpsGuard, 0, kMassEpsLanes, true>(a, sa, s)
+               : launchStrict<double, kEpsGuard, kPoly64Terms, kMassEpsLanes, true>(a, sa, s);
   }
   if (soft)
     return index ? launchStrict<float, kEpsGuard, kPolyMaxTerms, kMassEpsLanes, true>(a, sa, s)
