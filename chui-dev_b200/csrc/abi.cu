@@ -542,7 +542,7 @@ void applyConfig(Context& c, const chui_treepm_config& cfg) {
   c.cutoff = cfg.rcut_cells * c.spacing;
   const double t_cut = (c.cutoff * c.cutoff) / (4.0 * c.rs * c.rs) * (1.0 + 1.0e-5);
   c.poly = fitPoly(t_cut);
-  c.poly64 = fitPoly64(c.rs, c.cutoff);
+  c.poly64_fitted = false;
   c.dpoly = fitChebyshev(hostHp, t_cut);
   // H'' scales the quadrupole's second-derivative term only: 1e-5 suffices
   c.ddpoly = fitChebyshev(hostHpp, t_cut, 1.0e-5);

@@ -70,7 +70,8 @@ struct Context {
   int device = 0;
   double spacing = 0.0, rs = 0.0, cutoff = 0.0;
   PolyH poly;
-  PolyH64 poly64;  // H(t) for FP64 pairs
+  PolyH64 poly64;  // H(t) for FP64 pairs, fitted by the first walk that reads it
+  bool poly64_fitted = false;
   PolyH dpoly;   // H'(t): the adjoint walk and FP32 multipoles
   PolyH ddpoly;  // H''(t): FP32 quadrupoles
   std::string last_error;

@@ -816,6 +816,10 @@ int walkStrictRun(Context& c, WalkArgs& a, bool f64, bool tiny, cudaStream_t s) 
   const bool index = a.tx != nullptr;
   const bool soft = a.src_eps || a.tgt_eps;
   if (f64) {
+    if (!c.poly64_fitted) {
+      c.poly64 = fitPoly64(c.rs, c.cutoff);
+      c.poly64_fitted = true;
+    }
     for (int j = 0; j < kPoly64Terms; ++j) sa.h64[j] = c.poly64.c[j];
     sa.h64_scale = c.poly64.scale;
     sa.canonical = 1;

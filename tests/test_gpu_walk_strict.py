@@ -317,3 +317,42 @@ def test_fp64_coincident_and_close_pairs(away):
             alone = ~np.isin(rows, at[300:600]) & ~np.isin(rows, far)
             scale = size[alone] + np.median(size)
             assert (np.linalg.norm(got - ref[:, rows], axis=0)[alone] / scale).max() <= 1e-11
+
+
+def long_double_pairs(p, box, rs, rcut, eps):
+    """Short-range accelerations in long double, and the sums of m d K_soft and
+    m K_soft over each target's pairs."""
+    x, m, L = np.stack(p[:3], 1).astype(np.longdouble), p[3], np.array(box, np.longdouble)
+    acc, soft, slope = np.zeros(x.shape, np.longdouble), np.zeros(len(m)), np.zeros(len(m))
+    for i in range(len(m)):
+        d = x - x[i]
+        d -= L * np.rint(d / L)
+        r2 = (d * d).sum(1)
+        use = (r2 <= np.longdouble(rcut) ** 2) & (r2 > 0)
+        d, r2, mj = d[use], r2[use], m[use]
+        t = r2 / (4 * np.longdouble(rs) ** 2)
+        h, term = np.zeros_like(t), np.full_like(t, 1 / np.longdouble(3))
+        for k in range(1, 120):  # H(t) = (4/sqrt(pi)) e^-t sum_k (2t)^k / (3 5 ... (2k+3))
+            h, term = h + term, term * 2 * t / (2 * k + 3)
+        h *= 4 / np.sqrt(np.longdouble("3.14159265358979323846264338327950288")) * np.exp(-t)
+        k_soft = (r2 + np.longdouble(eps) ** 2) ** np.longdouble(-1.5)
+        acc[i] = ((mj * (k_soft - h / (8 * np.longdouble(rs) ** 3)))[:, None] * d).sum(0)
+        soft[i], slope[i] = float((mj * k_soft * np.sqrt(r2)).sum()), float((mj * k_soft).sum())
+    return acc.T, soft, slope
+
+
+def test_fp64_pairs_to_the_last_digits():
+    """The FP64 pairs alone, against long double: every pair within 4e-16 of its
+    K_soft part, offsets of up to 3 r_cut within 2^-53, sums of up to 2000 pairs.
+    set_config changes the polynomial with the cutoff."""
+    p = particles(2000, 23)
+    p[0][0] = p[0][1] + 1e-6  # one close pair
+    cell = (BOX[0] * BOX[1] * BOX[2]) ** (1 / 3) / 48
+    with ct.TreePmCoordinator(config(48, ct._abi.FP64, multipole_order=0, softening=0.002, short_range_only=1)) as s:
+        for cells in (6.25, 4.5):
+            s.set_config(config(48, ct._abi.FP64, multipole_order=0, softening=0.002, short_range_only=1, rcut_cells=cells))
+            r = s.solve_active_set(*p)
+            ref, soft, slope = long_double_pairs(p, BOX, 1.25 * cell, cells * cell, 0.002)
+            d = np.sqrt(((np.stack([np.asarray(r[k]) for k in ("ax", "ay", "az")]) - ref) ** 2).sum(0)).astype(float)
+            allow = 1.2e-15 * soft + 2.0 * slope * 3.0 * cells * cell * 2.0 ** -53
+            assert (d <= allow).all(), (d / allow).max()
