@@ -1,4 +1,7 @@
-// Short-range residual walk on the B200: the FLOP sink of the TreePM force.
+// Short-range residual walk: the reference's per-node walk in FP64 (walkKernel),
+// the adaptive policy's walk and the counting walks (walkFastKernel), the group
+// walk (groupWalkKernel), and the choice among these and walk_strict.cu, which is
+// the strict policy's production walk (walkRun).
 //
 // Reference: evaluateTargetAgainstLocalTree, tree_pm_coupling.cpp:4026-4272
 // (per-target DFS, periodic node metric, AABB cutoff prune, leaf pairs with
@@ -6,34 +9,31 @@
 // screened-quadrupole multipoles monopolePlusQuadrupoleAccelPeriodicReference
 // :743-827, children pushed in reverse octant order :916-925).
 //
-// Design: one warp walks 32 targets that are consecutive in tree order
-// (spatially coherent), sharing one DFS stack in shared memory. Every lane
-// makes the reference's own decision for every node it reaches, in FP64
-// (prune / leaf pairs / accept multipole / open); the warp descends into a
-// node's children when any lane opens it, and a lane that pruned or accepted
-// a node skips that node's subtree (nodes are numbered in preorder, so the
-// subtree is the index range [node, subtree_end)). Each lane therefore sees
-// exactly the nodes, pairs and multipoles of its own walk.
+// Design: one warp walks up to 32 targets that follow one another in tree order
+// (spatially coherent; under the adaptive policy the groups of walk_strict.cu),
+// sharing one DFS stack in shared memory. Every lane makes the reference's own
+// decision for every node it reaches (prune / leaf pairs / accept multipole /
+// open); the warp descends into a node's children when any lane opens it, and a
+// lane that pruned or accepted a node skips that node's subtree (nodes are
+// numbered in preorder, so the subtree is the index range [node, subtree_end)).
+// Each lane therefore sees exactly the nodes, pairs and multipoles of its own walk.
 //
-// Leaf sources are staged through shared memory per warp chunk of 32 and
-// broadcast to the lanes. Mixed precision: each source is stored as an FP32
-// offset from its leaf's FP64 centre; the target's offset to that centre is
-// formed in FP64 (the node metric) and rounded once, so the pair separation
-// is an FP32 difference of two small node-relative vectors. The residual
+// Mixed precision: each source is stored as an FP32 offset from its leaf's FP64
+// centre; offsets from the warp's frame are formed in FP64 and rounded once, so
+// the pair separation is an FP32 difference of two small vectors. The residual
 // kernel K = (r^2+eps^2)^-3/2 - H(t)/(8 r_s^3), t = r^2/(4 r_s^2), uses one
 // rsqrt and a polynomial for H fitted per configuration (no erf/exp per
-// pair). Per-leaf FP32 partial sums are added into FP64 accumulators. The
-// FP64 configuration evaluates the reference's formulas (source metric per
-// pair, erf/exp residual) unchanged.
+// pair). FP32 partial sums are added into FP64 accumulators. walkKernel
+// evaluates the reference's formulas (source metric per pair, erf/exp residual)
+// unchanged.
 //
-// With diagnostics on, the walk reproduces the reference's node counters
-// exactly. With diagnostics off (production), a small opened node is
-// evaluated as one block of sources instead of being descended: its lanes
-// get every source inside r_cut, which is the reference's pair set except
-// where a deeper node would have been accepted as a strict multipole (those
-// few are summed as pairs, which moves forces by far less than the mixed
-// precision does); the number of warp traversal steps drops several-fold,
-// and no counters are kept.
+// With diagnostics 1 the walk reproduces the reference's node counters exactly.
+// Otherwise a small opened node is evaluated as one block of sources instead of
+// being descended: its lanes get every source inside r_cut, which is the
+// reference's pair set except where a deeper node would have been accepted as a
+// strict multipole (those few are summed as pairs, which moves forces by far
+// less than the mixed precision does). Diagnostics 2 and a nearest-pair lane count
+// that walk; the strict policy without them takes walk_strict.cu.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -700,9 +700,9 @@ __global__ void __launch_bounds__(kWalkWarpsPerBlock * 32,
   constexpr bool kGroup = kMode == 3;
   constexpr bool kHistory = kMode != 0;
   constexpr int kList = kAdaptive ? kMultList : 1;
-  // sources per warp batch: longer for the strict walk (fewer flushes; 256
-  // against 64 took 224.1 to 219.8 ms at 256^3), the adaptive instances'
-  // shared memory (lane multipole lists) keeps them at 64 for occupancy
+  // sources per warp batch: 256 for the strict policy's counting and FP64
+  // instances (fewer flushes: 2 % at 256^3); the adaptive instances' shared
+  // memory (lane multipole lists) keeps them at 64 for occupancy
   constexpr int kQueueLen = kAdaptive ? kQueue : 4 * kQueue;
   static_assert(kQueueLen % 2 == 0, "the queue holds pairs of sources");
   __shared__ long long item_start_sm[kWalkWarpsPerBlock];
@@ -1567,8 +1567,8 @@ int walkRun(Context& c, int64_t nt, const uint32_t* active, const double* tx, co
   a.out_near = c.tree_near.as<double>();
   a.counters = c.walk_counters.as<unsigned long long>();
   a.work = c.work_counter.as<uint32_t>();
-  // per-block cycles for visit-range solves (FP64 walk, and the mixed walk's
-  // production instances: no diagnostics, every source a target, one mass)
+  // per-block cycles for visit-range solves (the strict production walk, the FP64
+  // walks, and the adaptive instances for every source a target and one mass)
   a.chunk_cost = record_cost ? c.walk_cost.as<float>() : nullptr;
   a.status = c.status.as<uint32_t>();
   a.poly = c.poly;

@@ -15,7 +15,7 @@ namespace chui {
 struct WalkArgs {
   int64_t nt;       // targets
   int64_t v0, v1;   // visit positions walked: [v0, v1) of the nt
-  float* chunk_cost;  // SM cycles spent per 32 visit positions (index base / 32), nullable
+  float* chunk_cost;  // SM cycles spent per 32 visit positions (index position / 32), nullable
   int out_compact;    // outputs at visit position - v0 (a visit-range solve) instead of the slot
   int64_t n;        // sources
   const uint32_t* order;   // visit position -> active slot

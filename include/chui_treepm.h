@@ -78,9 +78,13 @@ typedef struct {
                                                  counters; it still fills a requested nearest-pair lane.
                                                  1: the reference's per-node walk, traversal counters
                                                  equal to the reference's, nearest-pair r^2.
-                                                 2: the production walk with its own counters (its
-                                                 traversal's node visits and in-cutoff pairs) and the
-                                                 nearest-pair lane */
+                                                 2: subtree blocks as in production, with counters
+                                                 (node visits and in-cutoff pairs of that walk) and the
+                                                 nearest-pair lane. Under the strict policy this, and a
+                                                 nearest-pair lane with 0, run a walk of its own over
+                                                 runs of 32 targets: the production walk's forces to
+                                                 its rounding, at several times its cost below about
+                                                 two million particles */
   /* adaptive-relative policy (TreePmOptions, tree_pm_coupling.hpp:243-332) */
   int32_t adaptive_error_estimator;           /* CHUI_TREEPM_ESTIMATOR_*: treepm_adaptive_error_estimator */
   int32_t cutoff_node_policy;                 /* CHUI_TREEPM_CUTOFF_*: treepm_cutoff_node_policy */
@@ -218,9 +222,10 @@ int chui_treepm_visit_order(void *handle, int64_t begin, int64_t end, uint32_t *
 
 /* Device cycles the residual walk of the last successful solve spent on each
  * block of 32 visit positions: cost[k] covers positions begin + 32k ..
- * begin + 32k + 31 (SM clock cycles). Recorded by visit-range solves in FP64
- * and by the mixed walk's production form (diagnostics off, every source a
- * target, one mass for all sources); 0 elsewhere, where nothing was walked,
+ * begin + 32k + 31 (SM clock cycles). Recorded by visit-range solves: by every
+ * strict solve in production (diagnostics off), by FP64's other walks (the
+ * counting one: every source a target), and by the mixed adaptive walk where every
+ * source is a target and all have one mass; 0 elsewhere, where nothing was walked,
  * and for targets taken by the group walk. begin must be a multiple of 32;
  * cost holds ceil((end - begin) / 32) entries. No counterpart in the
  * reference; it lets a sharded solve cut the visit order into slices of equal
